@@ -69,11 +69,10 @@ cudaError_t launch_mortar(const MortarArgs& a, cudaStream_t s);
 
 // plain FP64 Euler path (stage_fp64.cu)
 cudaError_t setup_stage_euler64(const OpConsts& ops);
-cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool ind, bool rhs_only, cudaStream_t s);
+cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s);
 // conserved totals of the first n elements of an SoA state with element stride E
 cudaError_t launch_totals64(const double* u, const double* delta, int64_t E, int64_t n, int nv, double* part,
                             double* out, cudaStream_t s);
-int stage_smem_bytes64();
 // positivity repair of element states [n][nv][64] (one element per warp), ok[e] = admissible after
 cudaError_t launch_repair_states64(double* st, int64_t n, int nv, int mhd, int32_t* ok, cudaStream_t s);
 

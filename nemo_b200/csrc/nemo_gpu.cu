@@ -419,7 +419,7 @@ cudaError_t launch_stage_any(const StageArgs& a, bool rhs_only, cudaStream_t s) 
     }
     if (g.cfg.precision == NEMO_PREC_FP32)
         return launch_stage_euler32(a, blended(), rhs_only, s, g.tune_mode == 2 ? 4 : (g.tune_mode == 3 ? 16 : 8));
-    return launch_stage_euler64(a, blended(), blended(), rhs_only, s);
+    return launch_stage_euler64(a, blended(), rhs_only, s);
 }
 
 cudaError_t launch_stage(int st, cudaStream_t s) {

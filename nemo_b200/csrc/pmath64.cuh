@@ -12,6 +12,8 @@
 // Accuracy: within 3 ulp (log) and 2 ulp (exp), the order of the libraries they replace.
 #pragma once
 
+#include "ieee64.cuh"
+
 namespace nemo {
 
 constexpr double PM_LN2_HI = 0x1.62e42feep-1;            // ln 2 with a 32-bit mantissa
@@ -19,31 +21,41 @@ constexpr double PM_LN2_LO = 0x1.a39ef35793c76p-33;      // ln 2 - PM_LN2_HI
 constexpr double PM_INV_LN2 = 0x1.71547652b82fep+0;      // 1 / ln 2
 constexpr double PM_SQRT2 = 1.4142135623730951;
 
-__device__ __forceinline__ double plog64(double x) {
-    if (!(x > 0.0)) return x == 0.0 ? -__longlong_as_double(0x7ff0000000000000LL) : __longlong_as_double(0x7ff8000000000000LL);
-    if (x == __longlong_as_double(0x7ff0000000000000LL)) return x;
-    int shift = 0;
-    if (x < 2.2250738585072014e-308) { x = x * 18014398509481984.0; shift = 54; }  // 2^54
-    const long long b = __double_as_longlong(x);
-    int e = (int)((b >> 52) & 0x7ff) - 1023 - shift;
-    double m = __longlong_as_double((b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
+// Coefficients that are no short immediates: an operand from constant memory costs nothing, a literal
+// two register moves at each use.
+static __constant__ double PM_LOG[10] = {1.0 / 21.0, 1.0 / 19.0, 1.0 / 17.0, 1.0 / 15.0, 1.0 / 13.0,
+                                         1.0 / 11.0, 1.0 / 9.0,  1.0 / 7.0,  1.0 / 5.0,  1.0 / 3.0};
+
+__device__ __forceinline__ bool positive_normal64(double x) {
+    return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u;
+}
+
+// log of a positive normal number times 2^-shift, without a branch
+__device__ __forceinline__ double plog64_core(double x, int shift) {
+    int hi = __double2hiint(x);
+    int e = (hi >> 20) - 1023 - shift;
+    double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
     if (m > PM_SQRT2) { m = 0.5 * m; e = e + 1; }
-    const double s = (m - 1.0) / (m + 1.0);
+    const double s = div64(m - 1.0, m + 1.0);
     const double z = s * s;
-    double p = 1.0 / 21.0;
-    p = p * z + 1.0 / 19.0;
-    p = p * z + 1.0 / 17.0;
-    p = p * z + 1.0 / 15.0;
-    p = p * z + 1.0 / 13.0;
-    p = p * z + 1.0 / 11.0;
-    p = p * z + 1.0 / 9.0;
-    p = p * z + 1.0 / 7.0;
-    p = p * z + 1.0 / 5.0;
-    p = p * z + 1.0 / 3.0;
+    double p = PM_LOG[0];
+#pragma unroll
+    for (int i = 1; i < 10; ++i) p = p * z + PM_LOG[i];
     p = p * z + 1.0;
     const double lm = (2.0 * s) * p;
     const double de = (double)e;
     return de * PM_LN2_HI + (lm + de * PM_LN2_LO);
+}
+
+__device__ __forceinline__ double plog64(double x) {
+    int shift = 0;
+    if (!positive_normal64(x)) {
+        if (!(x > 0.0)) return x == 0.0 ? -__longlong_as_double(0x7ff0000000000000LL) : __longlong_as_double(0x7ff8000000000000LL);
+        if (x == __longlong_as_double(0x7ff0000000000000LL)) return x;
+        x = x * 18014398509481984.0;  // 2^54
+        shift = 54;
+    }
+    return plog64_core(x, shift);
 }
 
 __device__ __forceinline__ double pexp64(double y) {

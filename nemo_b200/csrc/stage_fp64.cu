@@ -1,20 +1,20 @@
 // stage_fp64.cu -- plain FP64 path: one fused kernel per LSRK stage (compiled with -fmad=false).
 //
-// One CTA owns EPC = 4 consecutive elements (a 2x2x1 block on a Morton-ordered brick) and runs
-// 48 threads per element, one per (direction d, line (a,b)).  Per stage and element it does what
-// the reference spreads over hook_pre_rk_timestep_300 and hook_mid_rk_timestep_500:
-//   1. TMA bulk copy (cp.async.bulk, mbarrier) of the 8 elements' SoA state into shared memory;
-//   2. per-node primitives (velocities, beta_d = rho/(2 p_d) per direction);
-//   3. the two face fluxes at the ends of the thread's line (kernel_fill_faceflux,
-//      source/kernel/mcfv/3d/kernel_flux_mod.f90:47-278; neighbour traces from shared memory
-//      when the neighbour is in the CTA, else from global memory);
-//   4. split-form flux differencing along the line, 6 node pairs in a fixed order, plus the
-//      surface lift, plus (alpha > 0) first-order FV subcells and the convex blend;
-//   5. the LSRK 5-4 register/state update (timedisc_probe, source/timedisc/rungekutta/
+// One CTA of 64 threads per element, one thread per node.  Per stage and element it does what the
+// reference spreads over hook_pre_rk_timestep_300 and hook_mid_rk_timestep_500:
+//   1. the element's state into shared memory, the 96 neighbour trace nodes (or 2:1 mortar flux rows)
+//      beside it by cp.async, in flight while
+//   2. the per-node primitives (velocities, beta_d = rho/(2 p_d) per direction) are computed;
+//   3. per direction, the 96 two-point fluxes of the split form (16 lines x 6 node pairs), the 32 face
+//      fluxes (kernel_fill_faceflux, source/kernel/mcfv/3d/kernel_flux_mod.f90:47-278) and, where
+//      alpha > 0, the 48 FV subcell fluxes, each an independent task of one thread with its result in
+//      shared memory; then each node sums its own pairs in a fixed order, the surface lift, the FV
+//      term and the convex blend;
+//   4. the LSRK 5-4 register/state update (timedisc_probe, source/timedisc/rungekutta/
 //      low-storage/4-5/timedisc_probe_mod.f90:7-39; rkstep_cb :19-49);
-//   6. the positivity repair (dgfv_repair_3d, source/kernel/mcfv/3d/kernel_validate_mod.f90:159-272);
-//   7. epilogue on the new state: the modal indicator for the next stage and, on the last
-//      stage, the per-element CFL bound for the next time step (kernel_timestep_mod.f90:348-394).
+//   5. the positivity repair (dgfv_repair_3d, source/kernel/mcfv/3d/kernel_validate_mod.f90:159-272);
+//   6. epilogue on the new state: the modal (or learned) indicator for the next stage and, on the
+//      last stage, the per-element CFL bound for the next time step (kernel_timestep_mod.f90:348-394).
 // The arithmetic follows oracle/nemo_oracle.cpp expression by expression, so the two agree to
 // the last bit except where log/exp enter.
 #include "common.cuh"
@@ -28,264 +28,208 @@ __constant__ OpConsts c_ops64;
 
 namespace {
 
-// Tile shape (compile-time knobs for tuning builds): elements per CTA and the minimum number of
-// resident CTAs per SM that __launch_bounds__ asks the register allocator for.  Measured on B200
-// (Sedov 32^3, plain FP64 stage, bit-identical results in every case): 8 elements x 1 CTA/SM at 168
-// registers 0.890 ms; 4 x 3 CTAs/SM at 96 registers 0.735 ms; 2 x 6 at 96 registers 0.764 ms;
-// 2 x 5 0.784 ms.  Three independent 192-thread CTAs per SM overlap one another's tile loads,
-// barriers and epilogues, which one 384-thread CTA cannot (barrier stalls were 2.0 per issue).
-#ifndef NEMO_FP64_EPC
-#define NEMO_FP64_EPC 4
-#endif
-#ifndef NEMO_FP64_MINB
-#define NEMO_FP64_MINB 3
-#endif
-constexpr int EPC = NEMO_FP64_EPC;   // elements per CTA
-constexpr int TPE = 48;              // threads per element
-constexpr int NT = EPC * TPE;        // 192 threads at 4 elements per CTA
+// One flux per thread instead of one line per thread: a thread that owned a whole line kept 4 x 5
+// accumulators and both face fluxes live across six inlined pair fluxes and five inlined Riemann solvers
+// (96 registers and 1 KB of spills, 18 warps per SM, instruction fetch the second largest stall).  As
+// tasks the kernel holds one copy of each flux, and no element waits for another of its CTA.  With the
+// quotients of ieee64.cuh, B200, us per stage, line form -> this: Sedov 32^3 664 -> 381 (0.16 of the FP64
+// FMA peak by algorithmic flops), Kelvin-Helmholtz forest of 24k elements 619 -> 340, 4^3 elements
+// 38 -> 19 (with the compiler's quotients and 16 warps per SM the task form alone was 727 at 32^3).
+// What bounds it now (ncu, Sedov 32^3): 242 M warp instructions at 56 % issue, of which 103 M FP64 (the
+// FP64 pipe 49 % busy); stalls per issue: dependent latency 2.3, CTA barriers 1.5, instruction fetch 1.2.
+// Resident elements per SM at 14 / 12 / 10 / 8 (72, 80, 96, 128 registers): 424 / 397 / 403 / 420 us
+// (measured with both logarithmic means of a pair under warp-wide branches).
+constexpr int TPE = 64;              // threads per element, one per node
 constexpr int V = 5;
-static_assert(NT / 32 >= EPC, "the repair runs one element per warp");
+constexpr int NPAIR = 6;             // node pairs of a line
+constexpr int FROW = NF + 4;         // row stride of the pair / subcell fluxes: the rows that a
+                                     // half-warp of nodes gathers from start 4 double-banks apart
+constexpr int CTAS64 = 12;           // resident CTAs (elements) per SM asked of the register allocator
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+// Shared memory of one element, in doubles
+constexpr int O_SU = 0;                          // [V][64] state
+constexpr int O_SP = O_SU + V * NP;              // [7][64] vx, vy, vz, beta_x, beta_y, beta_z, 1/rho
+constexpr int O_TR = O_SP + 7 * NP;              // [V][96] neighbour traces / mortar flux rows, then the
+                                                 // face fluxes in their places
+constexpr int O_SF = O_TR + V * 6 * NF;          // [V][6][FROW] pair fluxes of one direction
+constexpr int O_SV = O_SF + V * NPAIR * FROW;    // [V][3][FROW] subcell fluxes (blended kernels)
+constexpr int ELEM_PLAIN = O_SV;
+constexpr int ELEM_BLEND = O_SV + V * (NN - 1) * FROW;
+static_assert(O_SV - O_SP >= 6 * NP, "the epilogue's six node arrays fit behind the state");
+
+// Position of node n in the [64] arrays of state and primitives: the x and y digits are exclusive-ored
+// with a function of z (a GF(4) code), so that the 16 lines of each of the three directions fall on 16
+// different double-banks (in node order the x- and y-lines conflict four ways).
+__device__ __forceinline__ int swz(int z) { return (0x7e90 >> (4 * z)) & 15; }
+__device__ __forceinline__ int phys(int n) { return n ^ swz(n >> 4); }
+__device__ __forceinline__ int line_phys(int d, int ab, int i) {
+    if (d == 0) return ((4 * ab) ^ swz(ab >> 2)) ^ i;
+    if (d == 1) return (((ab & 3) | ((ab >> 2) << 4)) ^ swz(ab >> 2)) ^ (4 * i);
+    return (ab ^ swz(i)) | (i << 4);
 }
 
-// Bounded wait on an mbarrier phase; returns false if the bound expired.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned phase) {
-    unsigned addr = smem_u32(bar);
-    for (int it = 0; it < (1 << 24); ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(addr), "r"(phase) : "memory");
-        if (ok) return true;
-    }
-    return false;
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
 
-// Stage the tile's state (V arrays of nel*64 doubles, contiguous per variable) into smem: the issue
-// (barrier set-up, then thread 0 starts the bulk copies) and, after other work, the wait.
-__device__ __forceinline__ void tile_issue(double* su, const double* __restrict__ u, int64_t E, int64_t e0, int nel,
-                                          uint64_t* bar) {
-    if (threadIdx.x == 0) {
-        unsigned b = smem_u32(bar);
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned b = smem_u32(bar);
-        unsigned bytes = (unsigned)(nel * NP * 8);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes * V) : "memory");
-        for (int v = 0; v < V; ++v) {
-            const double* src = u + ((int64_t)v * E + e0) * NP;
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    smem_u32(su + v * EPC * NP)),
-                "l"(src), "r"(bytes), "r"(b)
-                : "memory");
-        }
-    }
-}
-
-__device__ __forceinline__ bool tile_wait(uint64_t* bar, Control* ctrl) {
-    bool ok = mbar_wait(bar, 0);
-    if (!ok) {
-        atomicOr(&ctrl->error, 1);
-        mbar_wait(bar, 0);  // second bounded wait for the copies still in flight
-    }
-    return ok;
-}
-
-
-// Epilogue on a state held in smem (the new state of a stage, or the uploaded state of a prepare
-// launch): the blending coefficient for the next stage (modal indicator, or learned indicator with
-// the modal one as fallback and judge) and, if requested, the per-element CFL bound.
 __device__ __forceinline__ double silu64(double x) { return x / (1.0 + pexp64(-x)); }
 
-__device__ void epilogue64(const StageArgs& a, const double* su, double* sp, unsigned long long (*s_lam)[3],
-                           int nel, int64_t e0, int tid, const OpConsts& k) {
-    __shared__ double s_am[EPC];
-    __shared__ int s_fb[EPC];
+// maximum over the warp by bit patterns (non-negative values; a NaN counts as the largest)
+__device__ __forceinline__ unsigned long long wmax64(double x) {
+    unsigned long long v = (unsigned long long)__double_as_longlong(x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Modal coefficients of the nodal values q (one per thread) into cm[64]: x and y inside a warp, z
+// across the element's two warps; t1, t2 are [64] scratch.
+__device__ __forceinline__ double modal64(double q, double* t1, double* t2, const double* vi, int n) {
+    const int x = n & 3, y = (n >> 2) & 3, z = n >> 4;
+    t1[n] = q;
+    __syncwarp();
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < NN; ++i) s = s + vi[x * NN + i] * t1[nidx(i, y, z)];
+    t2[n] = s;
+    __syncwarp();
+    s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NN; ++j) s = s + vi[y * NN + j] * t2[nidx(x, j, z)];
+    __syncwarp();
+    t1[n] = s;
+    __syncthreads();
+    s = 0.0;
+#pragma unroll
+    for (int k = 0; k < NN; ++k) s = s + vi[z * NN + k] * t1[nidx(x, y, k)];
+    return s;
+}
+
+// Epilogue on the state u of this thread's node (the new state of a stage, or the uploaded state of a
+// prepare launch): the blending coefficient for the next stage (modal indicator, or learned indicator
+// with the modal one as fallback and judge) and, if requested, the per-element CFL bound.  sp: scratch
+// of the element, six [64] arrays.  Sums run in the oracle's serial order.
+__device__ __forceinline__ void epilogue64(const StageArgs& a, const double* u, double* sp, const double* vi,
+                                           unsigned long long (*s_lam)[3], int64_t e, int n, const OpConsts& k) {
     Control* ctrl = a.ctrl;
-    const int64_t E = a.E;
-    (void)E;
+    const int lane = n & 31, w = n >> 5;
     if (a.alpha_out) {
-        const bool learned = a.mlp64 != nullptr;
-        double* q = sp;
-        double* t1 = sp + EPC * NP;
-        double* t2 = sp + 2 * EPC * NP;
-        const int nq = learned ? 3 : 1;   // modal coefficients of rho*p, then rho and p
-        for (int w = 0; w < nq; ++w) {
-            double* cm = sp + (3 + w) * EPC * NP;
-            for (int p = tid; p < nel * NP; p += NT) {
-                const int pel = p / NP, n = p % NP;
-                double uu[V];
-#pragma unroll
-                for (int v = 0; v < V; ++v) uu[v] = su[(v * EPC + pel) * NP + n];
-                q[pel * NP + n] = w == 0 ? uu[0] * pressure64(uu, k) : (w == 1 ? uu[0] : pressure64(uu, k));
-            }
-            __syncthreads();
-            for (int p = tid; p < nel * NP; p += NT) {
-                const int pel = p / NP, n = p % NP;
-                const int ai = n % NN, j = (n / NN) % NN, kk = n / NF;
-                double s = 0.0;
-#pragma unroll
-                for (int i = 0; i < NN; ++i) s = s + k.Vinv[ai * NN + i] * q[pel * NP + nidx(i, j, kk)];
-                t1[pel * NP + n] = s;
-            }
-            __syncthreads();
-            for (int p = tid; p < nel * NP; p += NT) {
-                const int pel = p / NP, n = p % NP;
-                const int ai = n % NN, bj = (n / NN) % NN, kk = n / NF;
-                double s = 0.0;
-#pragma unroll
-                for (int j = 0; j < NN; ++j) s = s + k.Vinv[bj * NN + j] * t1[pel * NP + nidx(ai, j, kk)];
-                t2[pel * NP + n] = s;
-            }
-            __syncthreads();
-            for (int p = tid; p < nel * NP; p += NT) {
-                const int pel = p / NP, n = p % NP;
-                const int ai = n % NN, bj = (n / NN) % NN, cc = n / NF;
-                double s = 0.0;
-#pragma unroll
-                for (int kk = 0; kk < NN; ++kk) s = s + k.Vinv[cc * NN + kk] * t2[pel * NP + nidx(ai, bj, kk)];
-                cm[pel * NP + n] = s;
-            }
-            __syncthreads();
-        }
-        double* feat = q;   // [EPC][12], the nodal scratch is dead now
-        if (tid < nel) {
-            const double* m = sp + 3 * EPC * NP + tid * NP;
-            double total = 0.0, clip1 = 0.0, clip2 = 0.0;
-            for (int cc = 0; cc < NN; ++cc)
-                for (int bj = 0; bj < NN; ++bj)
-                    for (int ai = 0; ai < NN; ++ai) {
-                        const double mv = m[nidx(ai, bj, cc)];
-                        const double e2 = mv * mv;
-                        total = total + e2;
-                        if (ai < NN - 1 && bj < NN - 1 && cc < NN - 1) clip1 = clip1 + e2;
-                        if (ai < NN - 2 && bj < NN - 2 && cc < NN - 2) clip2 = clip2 + e2;
-                    }
-            const double e1 = (total - clip1) / total;
-            const double e2 = (clip1 - clip2) / clip1;
-            const double energy = fmax(e1, e2);
+        double* e2 = sp + 2 * NP;   // [3][64]: squared modes, those of order < N, those of order < N-1
+        const double m = modal64(u[0] * pressure64(u, k), sp, sp + NP, vi, n);
+        const int top = max(max(n & 3, (n >> 2) & 3), n >> 4);
+        e2[n] = m * m;
+        e2[NP + n] = top < NN - 1 ? m * m : 0.0;
+        e2[2 * NP + n] = top < NN - 2 ? m * m : 0.0;
+        __syncthreads();
+        double am = 0.0;
+        if (w == 0) {
+            // one sum per lane 0..2, in mode order (the zeros change nothing)
+            const double* el = e2 + (lane < 3 ? lane : 0) * NP;
+            double s = 0.0;
+#pragma unroll 16
+            for (int p = 0; p < NP; ++p) s = s + el[p];
+            const double total = __shfl_sync(0xffffffffu, s, 0);
+            const double clip1 = __shfl_sync(0xffffffffu, s, 1);
+            const double clip2 = __shfl_sync(0xffffffffu, s, 2);
+            const double energy = fmax((total - clip1) / total, (clip1 - clip2) / clip1);
             double al = 1.0 / (1.0 + pexp64(k.ind_k * (energy - k.ind_T)));
             if (al < k.alpha_min) al = 0.0;
             else if (al > k.one_m_alpha_min) al = 1.0;
-            s_am[tid] = fmin(k.alpha_max, al);
-            int fb = 0;
-            if (learned) {
-                // positivity-risk check: min nodal rho or p below a tenth of the element mean
-                double rs = 0.0, ps = 0.0, rmin = 1e300, pmin = 1e300;
-                for (int n = 0; n < NP; ++n) {
-                    double uu[V];
-#pragma unroll
-                    for (int v = 0; v < V; ++v) uu[v] = su[(v * EPC + tid) * NP + n];
-                    const double pr = pressure64(uu, k);
-                    rs = rs + uu[0];
-                    ps = ps + pr;
-                    rmin = fmin(rmin, uu[0]);
-                    pmin = fmin(pmin, pr);
-                }
-                if (rmin < 0.1 * (rs / 64.0) || pmin < 0.1 * (ps / 64.0)) fb = 1;
-                for (int w = 0; w < 2; ++w) {
-                    const double* mw = sp + (4 + w) * EPC * NP + tid * NP;
-                    double tot = 0.0, Eo[6] = {0, 0, 0, 0, 0, 0};
-                    for (int cc = 0; cc < NN; ++cc)
-                        for (int bj = 0; bj < NN; ++bj)
-                            for (int ai = 0; ai < NN; ++ai) {
-                                const double mv = mw[nidx(ai, bj, cc)];
-                                const double ee = mv * mv;
-                                tot = tot + ee;
-                                const int ord[3] = {ai, bj, cc};
-#pragma unroll
-                                for (int d = 0; d < 3; ++d) {
-                                    if (ord[d] == NN - 1) Eo[2 * d] = Eo[2 * d] + ee;
-                                    if (ord[d] == NN - 2) Eo[2 * d + 1] = Eo[2 * d + 1] + ee;
-                                }
-                            }
-                    for (int i = 0; i < 6; ++i) {
-                        const double f = plog64(Eo[i] / tot + 1e-12);
-                        feat[tid * 12 + 6 * w + i] = f;
-                        const double x = f / 10.0 + 1.0;
-                        if (x < a.mlp64[MLP_NW + 6 * w + i] || x > a.mlp64[MLP_NW + 12 + 6 * w + i]) fb = 1;
-                    }
-                }
-            }
-            s_fb[tid] = fb;
+            am = fmin(k.alpha_max, al);
         }
-        __syncthreads();
-        if (learned) {
-            const double* W1 = a.mlp64;
-            const double* b1 = W1 + 32 * 12;
-            const double* W2 = b1 + 32;
-            const double* b2 = W2 + 32 * 32;
-            const double* W3 = b2 + 32;
-            double* h1 = t1;   // [EPC][32]
-            double* h2 = t2;
-            for (int p = tid; p < nel * 32; p += NT) {
-                const int pel = p / 32, j = p % 32;
-                double s = b1[j];
-                for (int i = 0; i < 12; ++i) s = s + W1[j * 12 + i] * (feat[pel * 12 + i] / 10.0 + 1.0);
-                h1[pel * 32 + j] = silu64(s);
-            }
+        if (a.mlp64 == nullptr) {
+            if (n == 0) a.alpha_out[e] = am;
+        } else {
+            // learned indicator: squared modes of rho and p, nodal rho and p, then warp 0 alone
+            double* er = sp + 3 * NP;
+            double* ep = sp + 4 * NP;
+            double* np = sp + 5 * NP;
+            const double pr = pressure64(u, k);
+            __syncthreads();   // the sums above are done with e2
+            const double mr = modal64(u[0], sp, sp + NP, vi, n);
             __syncthreads();
-            for (int p = tid; p < nel * 32; p += NT) {
-                const int pel = p / 32, j = p % 32;
-                double s = b2[j];
-                for (int i = 0; i < 32; ++i) s = s + W2[j * 32 + i] * h1[pel * 32 + i];
-                h2[pel * 32 + j] = silu64(s);
-            }
+            const double mp = modal64(pr, sp, sp + NP, vi, n);
+            er[n] = mr * mr;
+            ep[n] = mp * mp;
+            np[n] = pr;
             __syncthreads();
-            if (tid < nel) {
-                double z = W3[32];
-                for (int j = 0; j < 32; ++j) z = z + W3[j] * h2[tid * 32 + j];
-                double al = k.alpha_max / (1.0 + pexp64(-z));
-                if (al < k.alpha_min) al = 0.0;
-                const double am = s_am[tid];
-                if (s_fb[tid]) {
-                    atomicAdd(&ctrl->fallback, 1ull);
-                    al = am;
-                } else {
-                    atomicAdd(&ctrl->judge_sum, fabs(al - am));
-                    atomicAdd(&ctrl->judge_n, 1ull);
+            sp[n] = u[0];     // nodal rho (the transform scratch is dead)
+            __syncthreads();
+            if (w == 0) {
+                double* feat = sp + NP;      // [12]
+                double* h1 = sp + NP + 16;   // [32]
+                double* h2 = e2;             // [32]
+                int fb = 0;
+                // positivity-risk check: min nodal rho or p below a tenth of the element mean (lanes 0, 1)
+                if (lane < 2) {
+                    const double* q = lane == 0 ? sp : np;
+                    double s = 0.0, mn = 1e300;
+                    for (int p = 0; p < NP; ++p) {
+                        s = s + q[p];
+                        mn = fmin(mn, q[p]);
+                    }
+                    if (mn < 0.1 * (s / 64.0)) fb = 1;
                 }
-                a.alpha_out[e0 + tid] = al;
+                if (lane < 12) {   // one feature per lane: quantity, direction, order
+                    const int wq = lane / 6, i = lane % 6, d = i >> 1, want = NN - 1 - (i & 1);
+                    const double* mw = wq ? ep : er;
+                    double tot = 0.0, eo = 0.0;
+                    for (int p = 0; p < NP; ++p) {
+                        const double ee = mw[p];
+                        tot = tot + ee;
+                        if (((p >> (2 * d)) & 3) == want) eo = eo + ee;
+                    }
+                    const double f = plog64(eo / tot + 1e-12);
+                    feat[lane] = f;
+                    const double x = f / 10.0 + 1.0;
+                    if (x < a.mlp64[MLP_NW + lane] || x > a.mlp64[MLP_NW + 12 + lane]) fb = 1;
+                }
+                fb = __any_sync(0xffffffffu, fb);
+                const double* W1 = a.mlp64;
+                const double* b1 = W1 + 32 * 12;
+                const double* W2 = b1 + 32;
+                const double* b2 = W2 + 32 * 32;
+                const double* W3 = b2 + 32;
+                double s = b1[lane];
+                for (int i = 0; i < 12; ++i) s = s + W1[lane * 12 + i] * (feat[i] / 10.0 + 1.0);
+                h1[lane] = silu64(s);
+                __syncwarp();
+                s = b2[lane];
+                for (int i = 0; i < 32; ++i) s = s + W2[lane * 32 + i] * h1[i];
+                h2[lane] = silu64(s);
+                __syncwarp();
+                if (lane == 0) {
+                    double z = W3[32];
+                    for (int j = 0; j < 32; ++j) z = z + W3[j] * h2[j];
+                    double al = k.alpha_max / (1.0 + pexp64(-z));
+                    if (al < k.alpha_min) al = 0.0;
+                    if (fb) {
+                        atomicAdd(&ctrl->fallback, 1ull);
+                        al = am;
+                    } else {
+                        atomicAdd(&ctrl->judge_sum, fabs(al - am));
+                        atomicAdd(&ctrl->judge_n, 1ull);
+                    }
+                    a.alpha_out[e] = al;
+                }
             }
-        } else if (tid < nel) {
-            a.alpha_out[e0 + tid] = s_am[tid];
         }
     }
     if (a.epi_dt) {
-        for (int p = tid; p < nel * NP; p += NT) {
-            const int pel = p / NP, n = p % NP;
-            double uu[V];
 #pragma unroll
-            for (int v = 0; v < V; ++v) uu[v] = su[(v * EPC + pel) * NP + n];
-            double rr[V];
-#pragma unroll
-            for (int dd = 0; dd < 3; ++dd) {
-                rr[0] = uu[0];
-                rr[1] = uu[1 + dd];
-                rr[2] = uu[1 + (dd + 1) % 3];
-                rr[3] = uu[1 + (dd + 2) % 3];
-                rr[4] = uu[4];
-                const double lam = xlambda64(rr, k);
-                atomicMax(&s_lam[pel][dd], (unsigned long long)__double_as_longlong(lam));
-            }
+        for (int dd = 0; dd < 3; ++dd) {
+            const double rr[V] = {u[0], u[1 + dd], u[1 + (dd + 1) % 3], u[1 + (dd + 2) % 3], u[4]};
+            const unsigned long long lam = wmax64(xlambda64(rr, k));
+            if (lane == 0) s_lam[w][dd] = lam;
         }
         __syncthreads();
-        if (tid < nel) {
-            const int64_t pe = e0 + tid;
-            const double lf = __longlong_as_double((long long)s_lam[tid][0]);
-            const double lg = __longlong_as_double((long long)s_lam[tid][1]);
-            const double lh = __longlong_as_double((long long)s_lam[tid][2]);
-            const double dte = fmin(fmin(a.delta[pe * 3 + 0] / lf, a.delta[pe * 3 + 1] / lg), a.delta[pe * 3 + 2] / lh);
-            const int g = a.group ? a.group[pe] : 0;
+        if (n == 0) {
+            const double lf = __longlong_as_double((long long)max(s_lam[0][0], s_lam[1][0]));
+            const double lg = __longlong_as_double((long long)max(s_lam[0][1], s_lam[1][1]));
+            const double lh = __longlong_as_double((long long)max(s_lam[0][2], s_lam[1][2]));
+            const double dte = fmin(fmin(a.delta[e * 3 + 0] / lf, a.delta[e * 3 + 1] / lg), a.delta[e * 3 + 2] / lh);
+            const int g = a.group ? a.group[e] : 0;
             atomicMin(&ctrl->dtmin_bits[g], (unsigned long long)__double_as_longlong(dte));
             atomicMax(&ctrl->lmax_bits[g], (unsigned long long)__double_as_longlong(fmax(fmax(lf, lg), lh)));
         }
@@ -294,303 +238,257 @@ __device__ void epilogue64(const StageArgs& a, const double* su, double* sp, uns
 
 }  // namespace
 
-template <bool BLEND, bool IND, bool RHS_ONLY, bool FAST>
-__global__ void __launch_bounds__(NT, NEMO_FP64_MINB) k_stage_euler64(StageArgs a) {
-    extern __shared__ __align__(128) double smem[];
-    double* su = smem;                    // [V][EPC][64] state, later the new state
-    double* sp = su + V * EPC * NP;       // [6][EPC][64] vx,vy,vz,beta_x,beta_y,beta_z; later R_x
-    double* sR = sp + 6 * EPC * NP;       // [2][V][EPC][64] R_y, R_z
-    __shared__ uint64_t bar;
-    __shared__ double s_alpha[EPC];
-    __shared__ int s_bad[EPC];
-    __shared__ unsigned long long s_lam[EPC][3];
+template <bool BLEND, bool RHS_ONLY, bool FAST>
+__global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
+    extern __shared__ __align__(16) double smem[];
+    __shared__ double s_S[NN * NN], s_winv[NN], s_vi[NN * NN];   // operator rows, indexed per thread
+    __shared__ double s_alpha;
+    __shared__ unsigned long long s_lam[2][3];
+    __shared__ int s_bad;
+    __shared__ int32_t s_nbr[6];
 
     const OpConsts& k = c_ops64;
     Control* ctrl = a.ctrl;
     if (!RHS_ONLY && ctrl->done) return;
 
-    const int tid = threadIdx.x;
+    const int n = threadIdx.x, lane = n & 31, w = n >> 5;
     const int64_t E = a.E;
-    const int64_t e0 = a.E_begin + (int64_t)blockIdx.x * EPC;
-    const int nel = (int)min((int64_t)EPC, a.E_own - e0);
-
-    // the tile's bulk copy first, so that it is in flight while the blending coefficients are read
-    tile_issue(su, a.u_in, E, e0, nel, &bar);
-    if (tid < EPC) {
-        s_bad[tid] = 0;
-        s_lam[tid][0] = s_lam[tid][1] = s_lam[tid][2] = 0ull;
-        double al = 0.0;
-        if (IND && tid < nel) {
-            int64_t e = e0 + tid;
-            al = a.alpha_in[e];
-            if (a.smooth) {
-#pragma unroll
-                for (int f = 0; f < 6; ++f) {
-                    int32_t ne = a.nbr[e * 6 + f];
-                    if (ne >= 0) al = fmax(al, 0.5 * a.alpha_in[ne]);
-                }
-            }
-            if (a.alpha_used) a.alpha_used[e] = al;
-        }
-        s_alpha[tid] = al;
+    const int64_t e = a.E_begin + blockIdx.x;
+    if (n < NN * NN) {
+        s_S[n] = k.S[n];
+        s_vi[n] = k.Vinv[n];
+        if (n < NN) s_winv[n] = k.winv[n];
     }
-    // s_alpha, s_bad and s_lam become visible at the barrier after the primitives: the coefficient
-    // loads overlap the bulk copy instead of holding the whole CTA
-    if (!tile_wait(&bar, ctrl)) return;
+    double* const su = smem + O_SU;
+    double* const sp = smem + O_SP;
+    double* const tr = smem + O_TR;
+    double* const sF = smem + O_SF;
+    double* const sV = smem + O_SV;
+
+    double q[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
     if (a.prep_only) {
         __syncthreads();
-        epilogue64(a, su, smem + V * EPC * NP, s_lam, nel, e0, tid, k);
+        epilogue64(a, q, sp, s_vi, s_lam, e, n, k);
         return;
+    }
+
+    // neighbour traces (or mortar flux rows) of the 96 face nodes, asynchronously
+    for (int p = n; p < 6 * NF; p += TPE) {
+        const int f = p >> 4, ab = p & 15;
+        const int32_t ne = __ldg(a.nbr + e * 6 + f);
+        if (ab == 0) s_nbr[f] = ne;
+        if (ne >= 0) {
+            const double* g = a.u_in + (int64_t)ne * NP + line_node(f >> 1, ab & 3, ab >> 2, (f & 1) ? 0 : NN - 1);
+#pragma unroll
+            for (int v = 0; v < V; ++v) cp_async8(tr + v * 6 * NF + p, g + (int64_t)v * E * NP);
+        } else if (ne <= -2) {
+            const double* g = a.mflux + (int64_t)(-2 - ne) * V * NF + ab;
+#pragma unroll
+            for (int v = 0; v < V; ++v) cp_async8(tr + v * 6 * NF + p, g + v * NF);
+        }
+    }
+    if (!RHS_ONLY && a.stage > 0 && n < 4 * V)   // the register rows (four lines each), needed at the end
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.reg + ((int64_t)(n >> 2) * E + e) * NP + 16 * (n & 3)));
+    if (n == 0) s_bad = 0;
+    if (BLEND && w == 0) {   // blending coefficient, smoothed over the conforming neighbours
+        double al = 0.0;
+        if (lane == 6) al = a.alpha_in[e];
+        if (a.smooth && lane < 6) {
+            const int32_t ne = __ldg(a.nbr + e * 6 + lane);
+            if (ne >= 0) al = 0.5 * a.alpha_in[ne];
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) al = fmax(al, __shfl_xor_sync(0xffffffffu, al, o));
+        if (lane == 0) {
+            s_alpha = al;
+            if (a.alpha_used) a.alpha_used[e] = al;
+        }
     }
 
     // per-node primitives: velocities and, per direction d, beta_d = rho/(2 p_d) where p_d is the
     // pressure of the state rotated into direction d (the reference evaluates the two-point flux on
     // the rotated state, so the kinetic-energy sum runs in the rotated component order)
-    for (int p = tid; p < nel * NP; p += NT) {
-        int el = p / NP, n = p % NP;
-        double q[5];
+    const int pn = phys(n);
 #pragma unroll
-        for (int v = 0; v < V; ++v) q[v] = su[(v * EPC + el) * NP + n];
-        sp[(0 * EPC + el) * NP + n] = q[1] / q[0];
-        sp[(1 * EPC + el) * NP + n] = q[2] / q[0];
-        sp[(2 * EPC + el) * NP + n] = q[3] / q[0];
+    for (int v = 0; v < V; ++v) su[v * NP + pn] = q[v];
+    const Rcp64 ir = rcp64r(q[0]);
+    sp[6 * NP + pn] = ir.y;
 #pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-            double r[5] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
-            sp[((3 + dd) * EPC + el) * NP + n] = 0.5 * q[0] / pressure64(r, k);
-        }
+    for (int c = 0; c < 3; ++c) sp[c * NP + pn] = quot64(q[1 + c], ir);
+#pragma unroll
+    for (int dd = 0; dd < 3; ++dd) {
+        const double r[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
+        sp[(3 + dd) * NP + pn] = div64(0.5 * q[0], pressure64(r, ir, k));
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+    const double al = BLEND ? s_alpha : 0.0;
 
-    const int el = tid / TPE;
-    const int r = tid % TPE;
-    const int d = r / NF;
-    const int ab = r % NF;
-    const int la = ab & 3, lb = ab >> 2;
-    const bool active = el < nel;
-    const int64_t e = e0 + el;
-    // rotated component c (0..2) of the momentum/velocity -> original index (d + c) % 3
-    const int c0 = d, c1 = (d + 1) % 3, c2 = (d + 2) % 3;
-
-    double t[NN][V];  // direction-d contribution per line node, rotated frame
-    if (active) {
-        // ---- split-form volume flux differencing along the line
-        int idx[NN];
+    // The node's rhs terms, in the component order of the current direction: after each direction the
+    // momentum entries are rotated on, so that the loop stays rolled.
+    double R[V];
 #pragma unroll
-        for (int i = 0; i < NN; ++i) idx[i] = line_node(d, la, lb, i);
-#pragma unroll
-        for (int i = 0; i < NN; ++i)
-#pragma unroll
-            for (int v = 0; v < V; ++v) t[i][v] = 0.0;
-        const int PI_[6] = {0, 0, 0, 1, 1, 2};
-        const int PM_[6] = {1, 2, 3, 2, 3, 3};
-#pragma unroll
-        for (int pq = 0; pq < 6; ++pq) {
-            const int i = PI_[pq], m = PM_[pq];
+    for (int v = 0; v < V; ++v) R[v] = 0.0;
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        const int c0 = d, c1 = d == 2 ? 0 : d + 1, c2 = d == 0 ? 2 : d - 1;
+        const double *m0 = su + (1 + c0) * NP, *m1 = su + (1 + c1) * NP, *m2 = su + (1 + c2) * NP;   // momenta
+        constexpr int VEL = O_SP - NP, BETA = O_SP + 2 * NP;   // from a momentum to its velocity, to its beta
+        // ---- two-point fluxes, two pairs of the 16 lines at a time: warp 0 pairs 0, 1, 4, 5, warp 1 pairs 2, 3
+        //      and then the faces (all pairs on warp 0: 396 against 383 us per stage at Sedov 32^3)
+#pragma unroll 1
+        for (int g = w; g < 3; g += 2) {
+            const int pq = 2 * g + (lane >> 4), ab = lane & 15;
+            const int i = line_phys(d, ab, (0x211000 >> (4 * pq)) & 3), m = line_phys(d, ab, (0x332321 >> (4 * pq)) & 3);
             double F[V];
             if (!FAST && a.volume_flux == NEMO_VOLFLUX_CENTRAL) {
-                double ui[V], um[V];
-                ui[0] = su[(0 * EPC + el) * NP + idx[i]];
-                ui[1] = su[((1 + c0) * EPC + el) * NP + idx[i]];
-                ui[2] = su[((1 + c1) * EPC + el) * NP + idx[i]];
-                ui[3] = su[((1 + c2) * EPC + el) * NP + idx[i]];
-                ui[4] = su[(4 * EPC + el) * NP + idx[i]];
-                um[0] = su[(0 * EPC + el) * NP + idx[m]];
-                um[1] = su[((1 + c0) * EPC + el) * NP + idx[m]];
-                um[2] = su[((1 + c1) * EPC + el) * NP + idx[m]];
-                um[3] = su[((1 + c2) * EPC + el) * NP + idx[m]];
-                um[4] = su[(4 * EPC + el) * NP + idx[m]];
-                central64(ui, pressure64(ui, k), um, pressure64(um, k), F);
+                const double ui[V] = {su[i], m0[i], m1[i], m2[i], su[4 * NP + i]};
+                const double um[V] = {su[m], m0[m], m1[m], m2[m], su[4 * NP + m]};
+                central64(ui, um, F, k);
             } else {
-                Node5 ni, nm;
-                ni.rho = su[(0 * EPC + el) * NP + idx[i]];
-                ni.vn = sp[(c0 * EPC + el) * NP + idx[i]];
-                ni.vt1 = sp[(c1 * EPC + el) * NP + idx[i]];
-                ni.vt2 = sp[(c2 * EPC + el) * NP + idx[i]];
-                ni.beta = sp[((3 + d) * EPC + el) * NP + idx[i]];
-                nm.rho = su[(0 * EPC + el) * NP + idx[m]];
-                nm.vn = sp[(c0 * EPC + el) * NP + idx[m]];
-                nm.vt1 = sp[(c1 * EPC + el) * NP + idx[m]];
-                nm.vt2 = sp[(c2 * EPC + el) * NP + idx[m]];
-                nm.beta = sp[((3 + d) * EPC + el) * NP + idx[m]];
+                const Node5 ni = {su[i], sp[6 * NP + i], m0[VEL + i], m1[VEL + i], m2[VEL + i], m0[BETA + i]};
+                const Node5 nm = {su[m], sp[6 * NP + m], m0[VEL + m], m1[VEL + m], m2[VEL + m], m0[BETA + m]};
                 chandrashekar64(ni, nm, F, k);
             }
-            const double sim = k.S[i * NN + m], smi = k.S[m * NN + i];
+#pragma unroll
+            for (int v = 0; v < V; ++v) sF[(v * NPAIR + pq) * FROW + ab] = F[v];
+        }
+        // ---- Riemann fluxes: round 0 the two faces of the 16 lines (warp 1), rounds 1 and 2 the FV subcell
+        //      interfaces 0, 1 (warp 0) and 2 (half of warp 1)
+        const int rounds = BLEND && al > 0.0 ? 3 : 1;
+#pragma unroll 1
+        for (int rt = 1 - w; rt < rounds; rt += 2) {
+            const int hi = lane >> 4, ab = lane & 15;
+            if (rt == 2 && hi) break;
+            const double *pL, *pR;
+            int stL = NP, stR = NP;
+            int32_t ne = 0;
+            double* own_tr = tr + (2 * d + hi) * NF + ab;
+            if (rt == 0) {
+                ne = s_nbr[2 * d + hi];
+                const double* own = su + line_phys(d, ab, hi ? NN - 1 : 0);
+                const double* oth = ne == -1 ? own : own_tr;   // domain boundary: the own trace
+                const int sto = ne == -1 ? NP : 6 * NF;
+                pL = hi ? own : oth;
+                pR = hi ? oth : own;
+                stL = hi ? NP : sto;
+                stR = hi ? sto : NP;
+            } else {
+                const int qi = 2 * (rt - 1) + hi;
+                pL = su + line_phys(d, ab, qi);
+                pR = su + line_phys(d, ab, qi + 1);
+            }
+            const double uL[V] = {pL[0], pL[(1 + c0) * stL], pL[(1 + c1) * stL], pL[(1 + c2) * stL], pL[4 * stL]};
+            const double uR[V] = {pR[0], pR[(1 + c0) * stR], pR[(1 + c1) * stR], pR[(1 + c2) * stR], pR[4 * stR]};
+            double F[V];
+            riem64<FAST>(a.surface_flux, uL, uR, F, k);
+            if (rt == 0) {
+                if (ne > -2) {   // a mortar's flux row is there already
+#pragma unroll
+                    for (int v = 0; v < V; ++v) own_tr[v * 6 * NF] = F[v];
+                }
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; ++v) sV[(v * (NN - 1) + 2 * (rt - 1) + hi) * FROW + ab] = F[v];
+            }
+        }
+        __syncthreads();
+        // ---- the node's terms: its three pairs in ascending order of the other node, lift, FV, blend
+        const int pos = (n >> (2 * d)) & 3;
+        const int ab = d == 0 ? n >> 2 : (d == 1 ? (n & 3) | ((n >> 4) << 2) : n & 15);
+        const unsigned rows = (unsigned)(0x0542053104300210ull >> (16 * pos));   // pair rows of this position
+        double t[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) t[v] = 0.0;
+#pragma unroll
+        for (int mm = 0; mm < NN - 1; ++mm) {
+            const double s = s_S[pos * NN + mm + (mm >= pos ? 1 : 0)];
+            const double* f = sF + ((rows >> (4 * mm)) & 15) * FROW + ab;
+#pragma unroll
+            for (int v = 0; v < V; ++v) t[v] = t[v] + s * f[v * NPAIR * FROW];
+        }
+        const double wi = s_winv[pos];
+        const double* sS = tr + 2 * d * NF + ab;   // face fluxes of the line: [v][2][NF]
+        if (pos == 0) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) t[v] = t[v] + wi * (-sS[v * 6 * NF]);
+        }
+        if (pos == NN - 1) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) t[v] = t[v] + wi * sS[v * 6 * NF + NF];
+        }
+        if (BLEND && al > 0.0) {
+            const double* fl = pos == 0 ? sS : sV + (pos - 1) * FROW + ab;
+            const double* fr = pos == NN - 1 ? sS + NF : sV + pos * FROW + ab;
+            const int sl = pos == 0 ? 6 * NF : (NN - 1) * FROW, sr = pos == NN - 1 ? 6 * NF : (NN - 1) * FROW;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-                t[i][v] = t[i][v] + sim * F[v];
-                t[m][v] = t[m][v] + smi * F[v];
+                const double fv = wi * (fr[v * sr] - fl[v * sl]);
+                t[v] = (1.0 - al) * t[v] + al * fv;
             }
         }
-        // ---- surface fluxes at the two ends of the line (faces 2d, 2d+1 at (la,lb)), after the
-        //      volume pairs so that they are not live during the pair loop (fewer registers)
-        double Fs[2][V];
+        const double cd = __ldg(a.cdel + e * 3 + d);
+        double r[V];
 #pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            const int f = 2 * d + side;
-            const int own = line_node(d, la, lb, side ? NN - 1 : 0);
-            double uo[V], un[V];
-            uo[0] = su[(0 * EPC + el) * NP + own];
-            uo[1] = su[((1 + c0) * EPC + el) * NP + own];
-            uo[2] = su[((1 + c1) * EPC + el) * NP + own];
-            uo[3] = su[((1 + c2) * EPC + el) * NP + own];
-            uo[4] = su[(4 * EPC + el) * NP + own];
-            const int32_t ne = a.nbr[e * 6 + f];
-            if (ne <= -2) {  // 2:1 mortar face: flux row of the mortar kernel
-                const double* mf = a.mflux + (int64_t)(-2 - ne) * V * NF + ab;
-#pragma unroll
-                for (int v = 0; v < V; ++v) Fs[side][v] = mf[v * NF];
-                continue;
-            }
-            if (ne >= 0) {
-                const int nn = line_node(d, la, lb, side ? 0 : NN - 1);
-                const int64_t nl = (int64_t)ne - e0;
-                if (nl >= 0 && nl < nel) {
-                    const int nli = (int)nl;
-                    un[0] = su[(0 * EPC + nli) * NP + nn];
-                    un[1] = su[((1 + c0) * EPC + nli) * NP + nn];
-                    un[2] = su[((1 + c1) * EPC + nli) * NP + nn];
-                    un[3] = su[((1 + c2) * EPC + nli) * NP + nn];
-                    un[4] = su[(4 * EPC + nli) * NP + nn];
-                } else {
-                    const double* g = a.u_in;
-                    un[0] = __ldg(g + ((int64_t)0 * E + ne) * NP + nn);
-                    un[1] = __ldg(g + ((int64_t)(1 + c0) * E + ne) * NP + nn);
-                    un[2] = __ldg(g + ((int64_t)(1 + c1) * E + ne) * NP + nn);
-                    un[3] = __ldg(g + ((int64_t)(1 + c2) * E + ne) * NP + nn);
-                    un[4] = __ldg(g + ((int64_t)4 * E + ne) * NP + nn);
-                }
-            } else {
-#pragma unroll
-                for (int v = 0; v < V; ++v) un[v] = uo[v];
-            }
-            if (side) riem64<FAST>(a.surface_flux, uo, un, Fs[1], k);
-            else riem64<FAST>(a.surface_flux, un, uo, Fs[0], k);
-        }
-
-        // ---- surface lift at the line ends
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            t[0][v] = t[0][v] + k.winv[0] * (-Fs[0][v]);
-            t[NN - 1][v] = t[NN - 1][v] + k.winv[NN - 1] * Fs[1][v];
-        }
-        // ---- FV subcells and convex blend
-        if (BLEND) {
-            const double al = s_alpha[el];
-            if (al > 0.0) {
-                double Fl[V], Fr[V];
-#pragma unroll
-                for (int v = 0; v < V; ++v) Fl[v] = Fs[0][v];
-#pragma unroll
-                for (int i = 0; i < NN; ++i) {
-                    if (i < NN - 1) {
-                        double uL[V], uR[V];
-                        uL[0] = su[(0 * EPC + el) * NP + idx[i]];
-                        uL[1] = su[((1 + c0) * EPC + el) * NP + idx[i]];
-                        uL[2] = su[((1 + c1) * EPC + el) * NP + idx[i]];
-                        uL[3] = su[((1 + c2) * EPC + el) * NP + idx[i]];
-                        uL[4] = su[(4 * EPC + el) * NP + idx[i]];
-                        uR[0] = su[(0 * EPC + el) * NP + idx[i + 1]];
-                        uR[1] = su[((1 + c0) * EPC + el) * NP + idx[i + 1]];
-                        uR[2] = su[((1 + c1) * EPC + el) * NP + idx[i + 1]];
-                        uR[3] = su[((1 + c2) * EPC + el) * NP + idx[i + 1]];
-                        uR[4] = su[(4 * EPC + el) * NP + idx[i + 1]];
-                        riem64<FAST>(a.surface_flux, uL, uR, Fr, k);
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < V; ++v) Fr[v] = Fs[1][v];
-                    }
-#pragma unroll
-                    for (int v = 0; v < V; ++v) {
-                        double fv = k.winv[i] * (Fr[v] - Fl[v]);
-                        t[i][v] = (1.0 - al) * t[i][v] + al * fv;
-                        Fl[v] = Fr[v];
-                    }
-                }
-            }
-        }
+        for (int v = 0; v < V; ++v) r[v] = d == 0 ? cd * t[v] : R[v] + cd * t[v];
+        R[0] = r[0];
+        R[1] = r[2];
+        R[2] = r[3];
+        R[3] = r[1];
+        R[4] = r[4];
+        __syncthreads();
     }
-    __syncthreads();  // all reads of the primitives done: sp becomes R_x
-    if (active) {
-        const double cd = a.cdel[e * 3 + d];
-        double* R = d == 0 ? sp : sR + (d - 1) * V * EPC * NP;
-#pragma unroll
-        for (int i = 0; i < NN; ++i) {
-            const int n = line_node(d, la, lb, i);
-            R[(0 * EPC + el) * NP + n] = cd * t[i][0];
-            R[((1 + c0) * EPC + el) * NP + n] = cd * t[i][1];
-            R[((1 + c1) * EPC + el) * NP + n] = cd * t[i][2];
-            R[((1 + c2) * EPC + el) * NP + n] = cd * t[i][3];
-            R[(4 * EPC + el) * NP + n] = cd * t[i][4];
-        }
-    }
-    __syncthreads();
 
     // ---- rhs, LSRK register and state update
+    const int64_t g0 = e * NP + n;
+    if (RHS_ONLY) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) a.rhs_out[(int64_t)v * E * NP + g0] = -R[v];
+        return;
+    }
     const int st = a.stage;
     const double A = rk_a(st);
-    const double Cdt = rk_c(st) * ctrl->dt[0];
-    for (int p = tid; p < nel * NP; p += NT) {
-        const int pel = p / NP, n = p % NP;
-        const int64_t pe = e0 + pel;
-        const double cdt = a.group ? rk_c(st) * ctrl->dt[a.group[pe]] : Cdt;
-        bool ok = true;
-        // the node's register values are loaded before any is stored (interleaved, each load would
-        // wait for the previous store: the compiler cannot prove the addresses differ)
-        double rg[V];
+    const double cdt = rk_c(st) * ctrl->dt[a.group ? a.group[e] : 0];
+    double rg[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) rg[v] = (RHS_ONLY || st == 0) ? 0.0 : a.reg[((int64_t)v * E + pe) * NP + n];
+    for (int v = 0; v < V; ++v) rg[v] = st == 0 ? 0.0 : a.reg[(int64_t)v * E * NP + g0];
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int s = (v * EPC + pel) * NP + n;
-            const double Rv = (sp[s] + sR[s]) + sR[V * EPC * NP + s];
-            const double rhs = -Rv;
-            const int64_t g = ((int64_t)v * E + pe) * NP + n;
-            if (RHS_ONLY) {
-                a.rhs_out[g] = rhs;
-            } else {
-                const double rr = st == 0 ? rhs : A * rg[v] + rhs;
-                a.reg[g] = rr;
-                su[s] = su[s] + cdt * rr;
+    for (int v = 0; v < V; ++v) {
+        const double rhs = -R[v];
+        const double rr = st == 0 ? rhs : A * rg[v] + rhs;
+        a.reg[(int64_t)v * E * NP + g0] = rr;
+        q[v] = su[v * NP + pn] + cdt * rr;
+    }
+    if (a.positivity) {
+        if (!isvalid64(q, k)) s_bad = 1;
+        __syncthreads();
+        if (s_bad) {
+            // lanes 0..15 of warp 0 repair the element together on a copy in node order (same
+            // arithmetic and order as the serial dgfv_repair_3d)
+#pragma unroll
+            for (int v = 0; v < V; ++v) sF[v * NP + n] = q[v];
+            __syncthreads();
+            if (n < 16) {
+                const bool repaired = repair_elem16<1>(sF, 0, n, k);
+                if (!repaired && n == 0) atomicAdd(&ctrl->nbad, 1ull);
             }
-        }
-        if (!RHS_ONLY && a.positivity) {
-            double q[V];
+            __syncthreads();
 #pragma unroll
-            for (int v = 0; v < V; ++v) q[v] = su[(v * EPC + pel) * NP + n];
-            ok = isvalid64(q, k);
-            if (!ok) s_bad[pel] = 1;
+            for (int v = 0; v < V; ++v) q[v] = sF[v * NP + n];
         }
     }
-    if (RHS_ONLY) return;
-    __syncthreads();
-    {   // element w is repaired by lanes 0..15 of warp w together (same arithmetic and order as the
-        // serial dgfv_repair_3d, no call frame in this kernel)
-        const int w = tid >> 5, lane = tid & 31;
-        if (a.positivity && w < nel && lane < 16 && s_bad[w]) {
-            const bool repaired = repair_elem16<EPC>(su, w, lane, k);
-            if (!repaired && lane == 0) atomicAdd(&ctrl->nbad, 1ull);
-        }
-    }
-    __syncthreads();
     // ---- source term after the stage, then store the new state
-    for (int p = tid; p < nel * NP; p += NT) {
-        const int pel = p / NP, n = p % NP;
-        if (k.cool) {
-            double q[V];
+    if (k.cool) q[4] = cooled_energy64(q, k);
 #pragma unroll
-            for (int v = 0; v < V; ++v) q[v] = su[(v * EPC + pel) * NP + n];
-            su[(4 * EPC + pel) * NP + n] = cooled_energy64(q, k);
-        }
-#pragma unroll
-        for (int v = 0; v < V; ++v) a.u_out[((int64_t)v * E + e0 + pel) * NP + n] = su[(v * EPC + pel) * NP + n];
-    }
-    if (st == 4 && a.tick && blockIdx.x == 0 && tid == 0) {
+    for (int v = 0; v < V; ++v) a.u_out[(int64_t)v * E * NP + g0] = q[v];
+    if (st == 4 && a.tick && blockIdx.x == 0 && n == 0) {
         for (int g = 0; g < ctrl->ngroups; ++g) ctrl->t[g] = ctrl->t[g] + ctrl->dt[g];
         ctrl->steps += 1;
     }
 
-    epilogue64(a, su, sp, s_lam, nel, e0, tid, k);
+    epilogue64(a, q, sp, s_vi, s_lam, e, n, k);
 }
 
 // Conserved totals: per-element weighted sums in the oracle's order, then a serial sum per
@@ -622,38 +520,44 @@ __global__ void k_totals_sum64(const double* __restrict__ part, int64_t E, int n
 // ---------------------------------------------------------------------------------------------
 // launchers
 
-int stage_smem_bytes64() { return (V * EPC * NP + 6 * EPC * NP + 2 * V * EPC * NP) * (int)sizeof(double); }
+static int smem64(bool blend) { return (blend ? ELEM_BLEND : ELEM_PLAIN) * (int)sizeof(double); }
 
-cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool ind, bool rhs_only, cudaStream_t s) {
-    const int grid = (int)((a.E_own - a.E_begin + EPC - 1) / EPC);
-    if (grid <= 0) return cudaSuccess;
-    const int smem = stage_smem_bytes64();
-    (void)ind;
+cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s) {
+    if (a.E_own <= a.E_begin) return cudaSuccess;
+    const unsigned grid = (unsigned)(a.E_own - a.E_begin);
+    const int smem = smem64(blend);
     // the specialised kernel for HLLC faces and Chandrashekar pairs, the general one for the rest
     const bool fast = a.surface_flux == NEMO_SURFFLUX_HLLC && a.volume_flux == NEMO_VOLFLUX_CHANDRASHEKAR;
     if (rhs_only) {
-        if (blend) k_stage_euler64<true, true, true, false><<<grid, NT, smem, s>>>(a);
-        else k_stage_euler64<false, false, true, false><<<grid, NT, smem, s>>>(a);
+        if (blend) k_stage_euler64<true, true, false><<<grid, TPE, smem, s>>>(a);
+        else k_stage_euler64<false, true, false><<<grid, TPE, smem, s>>>(a);
     } else if (fast) {
-        if (blend) k_stage_euler64<true, true, false, true><<<grid, NT, smem, s>>>(a);
-        else k_stage_euler64<false, false, false, true><<<grid, NT, smem, s>>>(a);
+        if (blend) k_stage_euler64<true, false, true><<<grid, TPE, smem, s>>>(a);
+        else k_stage_euler64<false, false, true><<<grid, TPE, smem, s>>>(a);
     } else {
-        if (blend) k_stage_euler64<true, true, false, false><<<grid, NT, smem, s>>>(a);
-        else k_stage_euler64<false, false, false, false><<<grid, NT, smem, s>>>(a);
+        if (blend) k_stage_euler64<true, false, false><<<grid, TPE, smem, s>>>(a);
+        else k_stage_euler64<false, false, false><<<grid, TPE, smem, s>>>(a);
     }
     return cudaGetLastError();
 }
 
+// The largest carveout: twelve elements take 220 KB of an SM's shared memory, and the kernel reads
+// nothing twice through L1.
+template <typename K>
+static cudaError_t attrs64(K kernel, int smem) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return err;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
 cudaError_t setup_stage_euler64(const OpConsts& ops) {
-    const int smem = stage_smem_bytes64();
     cudaError_t err;
-    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<true, true, true, false>, dyn, smem)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<false, false, true, false>, dyn, smem)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<true, true, false, false>, dyn, smem)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<false, false, false, false>, dyn, smem)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<true, true, false, true>, dyn, smem)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_euler64<false, false, false, true>, dyn, smem)) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<true, true, false>, smem64(true))) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<false, true, false>, smem64(false))) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<true, false, false>, smem64(true))) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<false, false, false>, smem64(false))) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<true, false, true>, smem64(true))) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<false, false, true>, smem64(false))) != cudaSuccess) return err;
     return cudaMemcpyToSymbol(c_ops64, &ops, sizeof(OpConsts));
 }
 

@@ -1,0 +1,78 @@
+"""The plain FP64 stage kernel where its task layout and its own quotients could go wrong: meshes down to a
+single element that is its own neighbour, odd element counts, domain boundaries, 2:1 faces, both kernels
+(specialised and general) with and without blending; and states whose densities and pressures sit on and
+next to 1 and 2, where a reciprocal rounds next to a tie.  Everything is compared with the FP64 oracle bit
+for bit: the plain path's contract leaves no tolerance."""
+import numpy as np
+import pytest
+
+from nemo_b200 import abi, mesh, setups
+from nemo_b200.solver import Solver
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _fin():
+    yield
+    try:
+        abi.call("nemo_gpu_finalize")
+    except Exception:
+        pass
+
+
+MESHES = {
+    "one periodic element": lambda: mesh.brick(1),
+    "one open element": lambda: mesh.brick(1, periodic=(False,) * 3),
+    "2x1x1": lambda: mesh.brick(2, 1, 1),
+    "3x5x2, open in y": lambda: mesh.brick(3, 5, 2, periodic=(True, False, True)),
+    "forest": lambda: mesh.forest(2, lambda lvl, c, s: c[:, 1] < 0.5, max_level=1),
+}
+
+
+@pytest.mark.parametrize("blend", [False, True])
+@pytest.mark.parametrize("vf,sf", [(abi.VOLFLUX_CHANDRASHEKAR, abi.SURFFLUX_HLLC), (abi.VOLFLUX_CENTRAL, abi.SURFFLUX_RUSANOV)])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_steps_bit_exact(name, vf, sf, blend):
+    m = MESHES[name]()
+    # a density jump between neighbouring nodes makes alpha > 0 in part of the elements
+    u = setups.smooth_random(m, seed=5)
+    u[:, :, 17] *= 1.5
+    c = abi.default_cfg(volume_flux=vf, surface_flux=sf, indicator=abi.IND_MODAL if blend else abi.IND_NONE, positivity=1)
+    s = Solver(c, m)
+    o = orc.Oracle.for_mesh(c, m)
+    s.upload(u)
+    assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)) if blend else o.rhs(u))
+    t, n = s.run(nsteps=3)
+    ref, tr, nr, _ = o.run(u, nsteps=3)
+    assert t == tr and n == nr
+    assert np.array_equal(s.download(), ref)
+
+
+@pytest.mark.parametrize("sf", [abi.SURFFLUX_HLLC, abi.SURFFLUX_RUSANOV])
+@pytest.mark.parametrize("base", [0.5, 1.0, 2.0])
+def test_quotients_next_to_powers_of_two(base, sf):
+    """Densities and pressures within a few ulp of a power of two, from below (significands of all ones) and
+    from above, on nodes at rest and moving: every quotient of the fluxes meets its rounding ties."""
+    m = mesh.brick(4)
+    rng = np.random.default_rng(3)
+    shape = (m.E, 64)
+
+    def near(b):
+        x = np.full(shape, b)
+        k = rng.integers(-4, 5, size=shape)
+        for _ in range(4):
+            x = np.where(k > 0, np.nextafter(x, 9.0), np.where(k < 0, np.nextafter(x, 0.0), x))
+            k = k - np.sign(k)
+        return x
+
+    v = [np.where(rng.random(shape) < 0.5, 0.0, rng.choice([0.25, 1.0, 2.0 ** -30, -0.5], size=shape)) for _ in range(3)]
+    rho, p = near(base), near(base)
+    rho[: m.E // 2] = near(1.0)[: m.E // 2]
+    u = np.ascontiguousarray(setups.prim2cons(rho, v[0], v[1], v[2], p, 1.4))
+    c = abi.default_cfg(surface_flux=sf, indicator=abi.IND_MODAL)
+    s = Solver(c, m)
+    s.upload(u)
+    o = orc.Oracle.for_mesh(c, m)
+    assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)))
