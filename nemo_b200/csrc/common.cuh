@@ -65,6 +65,7 @@ struct OpConsts {
     double alpha_min, alpha_max, one_m_alpha_min;
     double repair_decr;
     double mu0;
+    double skm1;           // 1/(kappa-1)
     int cool;              // barotropic cooling after every stage
     double cool_rho;       // dens_critical
     double cool_ci;        // k_isothermal / (kappa - 1)

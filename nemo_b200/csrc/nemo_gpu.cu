@@ -681,6 +681,7 @@ int nemo_gpu_init(const nemo_cfg* cfg) {
     o.one_m_alpha_min = 1.0 - cfg->alpha_min;
     o.repair_decr = cfg->repair_decr;
     o.mu0 = cfg->mu0;
+    o.skm1 = 1.0 / o.km1;
     o.cool = cfg->source == NEMO_SOURCE_BAROTROPIC_COOLING ? 1 : 0;
     o.cool_rho = cfg->dens_critical;
     o.cool_ci = cfg->k_isothermal / (cfg->kappa - 1.0);

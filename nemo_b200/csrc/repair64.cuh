@@ -10,76 +10,9 @@ namespace nemo {
 // dgfv_repair_3d (source/kernel/mcfv/3d/kernel_validate_mod.f90:159-272) with N_NODES = 4: if a
 // node is inadmissible, squeeze 2x2x2 tiles of node means towards their mean in steps of
 // repair_decr until the tile means are admissible, first on the 8 octants (2^3 nodes each), then
-// node by node inside each octant.  su holds the tile's state [5][EPC][64]; one thread per element.
-template <int EPC>
-__device__ __noinline__ bool repair_elem(double* su, int el, const OpConsts& k) {
-    constexpr int V = 5;
-    auto at = [&](int v, int p) -> double& { return su[(v * EPC + el) * NP + p]; };
-    auto node_ok = [&](int p) {
-        double q[5];
-        for (int v = 0; v < V; ++v) q[v] = at(v, p);
-        return isvalid64(q, k);
-    };
-    bool ok = true;
-    for (int p = 0; p < NP; ++p) ok = ok && node_ok(p);
-    if (ok) return true;
-    for (int level = 1; level <= 2; ++level) {
-        int mm = 1 << (level - 1), nn = 1 << (2 - level);
-        double ws = 1.0 / (double)(nn * nn * nn);
-        for (int r = 0; r < mm; ++r)
-            for (int pp = 0; pp < mm; ++pp)
-                for (int q = 0; q < mm; ++q) {
-                    double tiles[8][V], means[V];
-                    for (int t = 0; t < 8; ++t)
-                        for (int v = 0; v < V; ++v) tiles[t][v] = 0.0;
-                    for (int v = 0; v < V; ++v)
-                        for (int kk = 0; kk < 2; ++kk)
-                            for (int jj = 0; jj < 2; ++jj)
-                                for (int ii = 0; ii < 2; ++ii)
-                                    for (int kx = (2 * r + kk) * nn; kx < (2 * r + kk + 1) * nn; ++kx)
-                                        for (int jx = (2 * pp + jj) * nn; jx < (2 * pp + jj + 1) * nn; ++jx)
-                                            for (int ix = (2 * q + ii) * nn; ix < (2 * q + ii + 1) * nn; ++ix) {
-                                                int t = ii + 2 * (jj + 2 * kk);
-                                                tiles[t][v] = tiles[t][v] + ws * at(v, nidx(ix, jx, kx));
-                                            }
-                    bool tv = true;
-                    for (int t = 0; t < 8; ++t) tv = tv && isvalid64(tiles[t], k);
-                    if (tv) continue;
-                    for (int v = 0; v < V; ++v) {
-                        double s = 0.0;
-                        for (int t = 0; t < 8; ++t) s = s + tiles[t][v];
-                        means[v] = 0.125 * s;
-                    }
-                    double hiles[8][V];
-                    for (int t = 0; t < 8; ++t)
-                        for (int v = 0; v < V; ++v) hiles[t][v] = tiles[t][v] - means[v];
-                    double squeeze = 1.0;
-                    while (squeeze > 0.0) {
-                        squeeze = fmax(0.0, squeeze - k.repair_decr);
-                        for (int t = 0; t < 8; ++t)
-                            for (int v = 0; v < V; ++v) tiles[t][v] = means[v] + squeeze * hiles[t][v];
-                        bool tv2 = true;
-                        for (int t = 0; t < 8; ++t) tv2 = tv2 && isvalid64(tiles[t], k);
-                        if (tv2) break;
-                    }
-                    for (int v = 0; v < V; ++v)
-                        for (int kx = 2 * r * nn; kx < (2 * r + 2) * nn; ++kx)
-                            for (int jx = 2 * pp * nn; jx < (2 * pp + 2) * nn; ++jx)
-                                for (int ix = 2 * q * nn; ix < (2 * q + 2) * nn; ++ix) {
-                                    int p = nidx(ix, jx, kx);
-                                    at(v, p) = means[v] + squeeze * (at(v, p) - means[v]);
-                                }
-                }
-    }
-    ok = true;
-    for (int p = 0; p < NP; ++p) ok = ok && node_ok(p);
-    return ok;
-}
-
-
-// The same repair done by the element's 16 threads together (a half-warp that calls it as a whole),
-// for V variables and an admissibility test valid(q):
-// no per-thread tile arrays, so it inlines without a call frame.  Level 1 squeezes the 8 octants
+// node by node inside each octant.  su holds the tile's state [V][EPC][64].  The element's 16 threads
+// (a half-warp that calls it as a whole) work together, for V variables and an admissibility test
+// valid(q): no per-thread tile arrays, so it inlines without a call frame.  Level 1 squeezes the 8 octants
 // (lanes 0..7, one octant each); level 2 squeezes the 8 nodes of each octant (lanes 0..7 and 8..15
 // take one octant each, four rounds).  Each lane sums its tile in the serial routine's node order,
 // the means run over the tiles in tile order, and all lanes of a block take the same squeeze steps.
@@ -167,72 +100,5 @@ __device__ __forceinline__ bool repair_elem16_mhd(double* su, int el, int lane, 
     return repair_coop16<EPC, 9>(su, el, lane, k.repair_decr,
                                  [&](const double* q) { return m_isvalid<double>(q, k.kappa, k.mu0); });
 }
-
-// The same repair for the 9 GLM-MHD variables (MHD pressure in the admissibility check).
-template <int EPC>
-__device__ __noinline__ bool repair_elem_mhd(double* su, int el, const OpConsts& k) {
-    constexpr int V = 9;
-    auto at = [&](int v, int p) -> double& { return su[(v * EPC + el) * NP + p]; };
-    auto node_ok = [&](int p) {
-        double q[9];
-        for (int v = 0; v < V; ++v) q[v] = at(v, p);
-        return m_isvalid(q, k.kappa, k.mu0);
-    };
-    bool ok = true;
-    for (int p = 0; p < NP; ++p) ok = ok && node_ok(p);
-    if (ok) return true;
-    for (int level = 1; level <= 2; ++level) {
-        int mm = 1 << (level - 1), nn = 1 << (2 - level);
-        double ws = 1.0 / (double)(nn * nn * nn);
-        for (int r = 0; r < mm; ++r)
-            for (int pp = 0; pp < mm; ++pp)
-                for (int q = 0; q < mm; ++q) {
-                    double tiles[8][V], means[V];
-                    for (int t = 0; t < 8; ++t)
-                        for (int v = 0; v < V; ++v) tiles[t][v] = 0.0;
-                    for (int v = 0; v < V; ++v)
-                        for (int kk = 0; kk < 2; ++kk)
-                            for (int jj = 0; jj < 2; ++jj)
-                                for (int ii = 0; ii < 2; ++ii)
-                                    for (int kx = (2 * r + kk) * nn; kx < (2 * r + kk + 1) * nn; ++kx)
-                                        for (int jx = (2 * pp + jj) * nn; jx < (2 * pp + jj + 1) * nn; ++jx)
-                                            for (int ix = (2 * q + ii) * nn; ix < (2 * q + ii + 1) * nn; ++ix) {
-                                                int t = ii + 2 * (jj + 2 * kk);
-                                                tiles[t][v] = tiles[t][v] + ws * at(v, nidx(ix, jx, kx));
-                                            }
-                    bool tv = true;
-                    for (int t = 0; t < 8; ++t) tv = tv && m_isvalid(tiles[t], k.kappa, k.mu0);
-                    if (tv) continue;
-                    for (int v = 0; v < V; ++v) {
-                        double s = 0.0;
-                        for (int t = 0; t < 8; ++t) s = s + tiles[t][v];
-                        means[v] = 0.125 * s;
-                    }
-                    double hiles[8][V];
-                    for (int t = 0; t < 8; ++t)
-                        for (int v = 0; v < V; ++v) hiles[t][v] = tiles[t][v] - means[v];
-                    double squeeze = 1.0;
-                    while (squeeze > 0.0) {
-                        squeeze = fmax(0.0, squeeze - k.repair_decr);
-                        for (int t = 0; t < 8; ++t)
-                            for (int v = 0; v < V; ++v) tiles[t][v] = means[v] + squeeze * hiles[t][v];
-                        bool tv2 = true;
-                        for (int t = 0; t < 8; ++t) tv2 = tv2 && m_isvalid(tiles[t], k.kappa, k.mu0);
-                        if (tv2) break;
-                    }
-                    for (int v = 0; v < V; ++v)
-                        for (int kx = 2 * r * nn; kx < (2 * r + 2) * nn; ++kx)
-                            for (int jx = 2 * pp * nn; jx < (2 * pp + 2) * nn; ++jx)
-                                for (int ix = 2 * q * nn; ix < (2 * q + 2) * nn; ++ix) {
-                                    int p = nidx(ix, jx, kx);
-                                    at(v, p) = means[v] + squeeze * (at(v, p) - means[v]);
-                                }
-                }
-    }
-    ok = true;
-    for (int p = 0; p < NP; ++p) ok = ok && node_ok(p);
-    return ok;
-}
-
 
 }  // namespace nemo

@@ -83,6 +83,37 @@ __device__ __forceinline__ unsigned long long wmax64(double x) {
     return v;
 }
 
+// The element's blending coefficient, smoothed over its conforming neighbours (warp 0).
+__device__ __forceinline__ void smooth_alpha64(const StageArgs& a, int64_t e, int lane, double* s_alpha) {
+    double al = 0.0;
+    if (lane == 6) al = a.alpha_in[e];
+    if (a.smooth && lane < 6) {
+        const int32_t ne = __ldg(a.nbr + e * 6 + lane);
+        if (ne >= 0) al = 0.5 * a.alpha_in[ne];
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) al = fmax(al, __shfl_xor_sync(0xffffffffu, al, o));
+    if (lane == 0) {
+        *s_alpha = al;
+        if (a.alpha_used) a.alpha_used[e] = al;
+    }
+}
+
+// state of the node at index i rotated into a direction whose momenta start at m0, m1, m2 (the magnetic
+// field four variables further on); st: stride of the variables
+__device__ __forceinline__ void load_rot64(const double* u, const double* m0, const double* m1, const double* m2, int st,
+                                           int i, double* r) {
+    r[0] = u[i];
+    r[1] = m0[i];
+    r[2] = m1[i];
+    r[3] = m2[i];
+    r[4] = u[4 * st + i];
+    r[5] = m0[4 * st + i];
+    r[6] = m1[4 * st + i];
+    r[7] = m2[4 * st + i];
+    r[8] = u[8 * st + i];
+}
+
 // Modal coefficients of the nodal values q (one per thread) into cm[64]: x and y inside a warp, z
 // across the element's two warps; t1, t2 are [64] scratch.
 __device__ __forceinline__ double modal64(double q, double* t1, double* t2, const double* vi, int n) {
@@ -106,17 +137,20 @@ __device__ __forceinline__ double modal64(double q, double* t1, double* t2, cons
     return s;
 }
 
-// Epilogue on the state u of this thread's node (the new state of a stage, or the uploaded state of a
-// prepare launch): the blending coefficient for the next stage (modal indicator, or learned indicator
-// with the modal one as fallback and judge) and, if requested, the per-element CFL bound.  sp: scratch
-// of the element, six [64] arrays.  Sums run in the oracle's serial order.
-__device__ __forceinline__ void epilogue64(const StageArgs& a, const double* u, double* sp, const double* vi,
-                                           unsigned long long (*s_lam)[3], int64_t e, int n, const OpConsts& k) {
+// Epilogue on this thread's node of density rho and pressure pr (of the new state of a stage, or of the
+// uploaded state of a prepare launch): the blending coefficient for the next stage (modal indicator, or
+// learned indicator with the modal one as fallback and judge) and, if requested, the per-element CFL bound
+// from the wave speeds lambda(d).  sp: scratch of the element, six [64] arrays.  Sums run in the oracle's
+// serial order.
+template <typename Lambda>
+__device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, double pr, double* sp, const double* vi,
+                                           unsigned long long (*s_lam)[4], int64_t e, int n, const OpConsts& k,
+                                           Lambda lambda) {
     Control* ctrl = a.ctrl;
     const int lane = n & 31, w = n >> 5;
     if (a.alpha_out) {
         double* e2 = sp + 2 * NP;   // [3][64]: squared modes, those of order < N, those of order < N-1
-        const double m = modal64(u[0] * pressure64(u, k), sp, sp + NP, vi, n);
+        const double m = modal64(rho * pr, sp, sp + NP, vi, n);
         const int top = max(max(n & 3, (n >> 2) & 3), n >> 4);
         e2[n] = m * m;
         e2[NP + n] = top < NN - 1 ? m * m : 0.0;
@@ -145,16 +179,15 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, const double* u, 
             double* er = sp + 3 * NP;
             double* ep = sp + 4 * NP;
             double* np = sp + 5 * NP;
-            const double pr = pressure64(u, k);
             __syncthreads();   // the sums above are done with e2
-            const double mr = modal64(u[0], sp, sp + NP, vi, n);
+            const double mr = modal64(rho, sp, sp + NP, vi, n);
             __syncthreads();
             const double mp = modal64(pr, sp, sp + NP, vi, n);
             er[n] = mr * mr;
             ep[n] = mp * mp;
             np[n] = pr;
             __syncthreads();
-            sp[n] = u[0];     // nodal rho (the transform scratch is dead)
+            sp[n] = rho;     // nodal rho (the transform scratch is dead)
             __syncthreads();
             if (w == 0) {
                 double* feat = sp + NP;      // [12]
@@ -219,8 +252,7 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, const double* u, 
     if (a.epi_dt) {
 #pragma unroll
         for (int dd = 0; dd < 3; ++dd) {
-            const double rr[V] = {u[0], u[1 + dd], u[1 + (dd + 1) % 3], u[1 + (dd + 2) % 3], u[4]};
-            const unsigned long long lam = wmax64(xlambda64(rr, k));
+            const unsigned long long lam = wmax64(lambda(dd));
             if (lane == 0) s_lam[w][dd] = lam;
         }
         __syncthreads();
@@ -243,7 +275,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
     extern __shared__ __align__(16) double smem[];
     __shared__ double s_S[NN * NN], s_winv[NN], s_vi[NN * NN];   // operator rows, indexed per thread
     __shared__ double s_alpha;
-    __shared__ unsigned long long s_lam[2][3];
+    __shared__ unsigned long long s_lam[2][4];
     __shared__ int s_bad;
     __shared__ int32_t s_nbr[6];
 
@@ -268,9 +300,15 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
     double q[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
+    auto epilogue = [&]() {
+        epilogue64(a, q[0], pressure64(q, k), sp, s_vi, s_lam, e, n, k, [&](int dd) {
+            const double rr[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
+            return xlambda64(rr, k);
+        });
+    };
     if (a.prep_only) {
         __syncthreads();
-        epilogue64(a, q, sp, s_vi, s_lam, e, n, k);
+        epilogue();
         return;
     }
 
@@ -292,20 +330,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
     if (!RHS_ONLY && a.stage > 0 && n < 4 * V)   // the register rows (four lines each), needed at the end
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.reg + ((int64_t)(n >> 2) * E + e) * NP + 16 * (n & 3)));
     if (n == 0) s_bad = 0;
-    if (BLEND && w == 0) {   // blending coefficient, smoothed over the conforming neighbours
-        double al = 0.0;
-        if (lane == 6) al = a.alpha_in[e];
-        if (a.smooth && lane < 6) {
-            const int32_t ne = __ldg(a.nbr + e * 6 + lane);
-            if (ne >= 0) al = 0.5 * a.alpha_in[ne];
-        }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) al = fmax(al, __shfl_xor_sync(0xffffffffu, al, o));
-        if (lane == 0) {
-            s_alpha = al;
-            if (a.alpha_used) a.alpha_used[e] = al;
-        }
-    }
+    if (BLEND && w == 0) smooth_alpha64(a, e, lane, &s_alpha);
 
     // per-node primitives: velocities and, per direction d, beta_d = rho/(2 p_d) where p_d is the
     // pressure of the state rotated into direction d (the reference evaluates the two-point flux on
@@ -488,7 +513,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
         ctrl->steps += 1;
     }
 
-    epilogue64(a, q, sp, s_vi, s_lam, e, n, k);
+    epilogue();
 }
 
 // Conserved totals: per-element weighted sums in the oracle's order, then a serial sum per
@@ -569,40 +594,6 @@ cudaError_t launch_totals64(const double* u, const double* delta, int64_t E, int
 }
 
 
-// ---- GLM-MHD stage (double flux arithmetic).  Tile of the plain form: 4 elements (64 threads) with
-// at least 4 CTAs per SM at the full 255 registers (Orszag-Tang 64^3, B200: 12.81 ms per stage against
-// 13.21 ms for 8 elements x 1-2 CTAs/SM; 2 elements x 8 CTAs 12.81 ms; 4 x 5 at 168 registers
-// 15.89 ms; bit-identical results).  The FP32 form keeps its 8-element tile (stage_fp32.cu).
-#ifndef NEMO_MHD_EPC
-#define NEMO_MHD_EPC 4
-#endif
-#ifndef NEMO_MHD64_MINB
-#define NEMO_MHD64_MINB 4
-#endif
-#define NEMO_MHD_OPS c_ops64
-}  // namespace nemo
-#include "stage_mhd.cuh"
-namespace nemo {
-#undef NEMO_MHD_OPS
-
-// state, rhs rows and the subcell interface fluxes of each thread's line
-int stage_smem_bytes_mhd64() {
-    return mhd::V * mhd::EPC * (NP * (int)sizeof(double) + mhd::SPM * (int)sizeof(double)) +
-           (NN - 1) * mhd::V * mhd::NT * (int)sizeof(double);
-}
-
-cudaError_t setup_stage_mhd64() {
-    const int smem = stage_smem_bytes_mhd64();
-    cudaError_t err;
-    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((err = cudaFuncSetAttribute(k_stage_mhd<double, true, true, false>, dyn, smem))) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_mhd<double, false, true, false>, dyn, smem))) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_mhd<double, true, false, false>, dyn, smem))) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_mhd<double, false, false, false>, dyn, smem))) return err;
-    if ((err = cudaFuncSetAttribute(k_stage_mhd<double, true, false, true>, dyn, smem))) return err;
-    return cudaFuncSetAttribute(k_stage_mhd<double, false, false, true>, dyn, smem);
-}
-
 // Positivity repair of element states held outside the library (the per-quad kernel_repair of a
 // host, source/kernel/mcfv/3d/kernel_validate_mod.f90:27-157): one warp per element [nv][64] (the
 // Fortran state(n,n,n,nv) layout); if a node is inadmissible, lanes 0..15 run the cooperative
@@ -640,23 +631,7 @@ cudaError_t launch_repair_states64(double* st, int64_t n, int nv, int mhd, int32
     return cudaGetLastError();
 }
 
-cudaError_t launch_stage_mhd64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s) {
-    const int grid = (int)((a.E_own - a.E_begin + mhd::EPC - 1) / mhd::EPC);
-    if (grid <= 0) return cudaSuccess;
-    const int smem = stage_smem_bytes_mhd64();
-    // the specialised kernel for HLLD faces and the EC pair flux, the general one for the rest
-    const bool fast = a.surface_flux == NEMO_SURFFLUX_HLLD && a.volume_flux == NEMO_VOLFLUX_EC_MHD;
-    if (rhs_only) {
-        if (blend) k_stage_mhd<double, true, true, false><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<double, false, true, false><<<grid, mhd::NT, smem, s>>>(a);
-    } else if (fast) {
-        if (blend) k_stage_mhd<double, true, false, true><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<double, false, false, true><<<grid, mhd::NT, smem, s>>>(a);
-    } else {
-        if (blend) k_stage_mhd<double, true, false, false><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<double, false, false, false><<<grid, mhd::NT, smem, s>>>(a);
-    }
-    return cudaGetLastError();
-}
-
 }  // namespace nemo
+
+// ---- GLM-MHD stage
+#include "stage_mhd64.cuh"

@@ -1,11 +1,10 @@
-// stage_mhd.cuh -- fused LSRK stage for GLM-MHD (9 variables), templated on the flux arithmetic.
+// stage_mhd.cuh -- fused LSRK stage for GLM-MHD (9 variables), FP32-bulk form (the plain FP64 form is
+// stage_mhd64.cuh).
 //
-// Included by stage_fp64.cu (R = double, -fmad=false: bit-identical to the oracle) and by
-// stage_fp32.cu (R = float, fast math; state, register, update, repair and reductions stay FP64).
-// One CTA = EPC elements (8 for the FP32 form, 4 for the plain FP64 form), 16 threads per element;
-// thread (a,b) owns the x-, y- and z-lines through (a,b) and adds its direction terms into one
-// shared rhs array (x, then y, then z), which keeps the oracle's summation order.  Two kernels per
-// form: a general one (flux kinds chosen at run time) and one specialised to HLLD + EC.  Per line:
+// Included by stage_fp32.cu (R = float, fast math; state, register, update, repair and reductions stay
+// FP64).  One CTA = 8 elements, 16 threads per element; thread (a,b) owns the x-, y- and z-lines through
+// (a,b) and adds its direction terms into one shared rhs array (x, then y, then z).  Two kernels: a
+// general one (flux kinds chosen at run time) and one specialised to HLLD + EC.  Per line:
 // surface flux (HLLD or Rusanov) + the element's own-side
 // non-conservative Powell/GLM term at both ends, 6 node pairs of EC flux (Derigs) + non-conservative
 // term in flux-differencing form, the lift, and (alpha > 0) FV subcells with the same interface
@@ -24,18 +23,9 @@
 namespace nemo {
 namespace mhd {
 
-// Tile shape (compile-time knobs for tuning builds): elements per CTA (16 threads each) and, per
-// form, the minimum number of resident CTAs per SM asked of the register allocator.
-#ifndef NEMO_MHD_EPC
-#define NEMO_MHD_EPC 8
-#endif
-#ifndef NEMO_MHD64_MINB
-#define NEMO_MHD64_MINB 1
-#endif
-#ifndef NEMO_MHD32_MINB
+// Tile shape: elements per CTA (16 threads each) and the resident CTAs per SM asked of the register allocator
 #define NEMO_MHD32_MINB 3
-#endif
-constexpr int EPC = NEMO_MHD_EPC;
+constexpr int EPC = 8;
 constexpr int NT = 16 * EPC;
 constexpr int V = 9;
 // element stride of the rhs array: 6 words of padding move the two elements of a warp onto
@@ -151,9 +141,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
     Control* ctrl = a.ctrl;
     const R kap = (R)k.kappa, mu0 = (R)k.mu0;
     if (a.alpha_out) {
-        const R* W = nullptr;
-        if (sizeof(R) == 8) W = reinterpret_cast<const R*>(a.mlp64);
-        else W = reinterpret_cast<const R*>(a.mlp32);
+        const R* W = a.mlp32;
         const bool learned = W != nullptr;
         R* q = scr;
         R* t1 = scr + EPC * NP;
@@ -199,7 +187,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
             __syncthreads();
         }
         R* feat = q;
-        if constexpr (sizeof(R) == 4) {
+        {
             // FP32 form: the element's 16 threads share the sums (modes / nodes lane + 16 q)
             const int pel = tid >> 4, lane = tid & 15;
             const bool act = pel < nel;
@@ -280,66 +268,6 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
                 fb = fb || oob != 0u;
             }
             if (act && lane == 0) s_fb[pel] = fb ? 1 : 0;
-        } else {
-            if (tid < nel) {
-                const R* m = scr + 3 * EPC * NP + tid * NP;
-                R total = R(0.0), clip1 = R(0.0), clip2 = R(0.0);
-                for (int cc = 0; cc < NN; ++cc)
-                    for (int bj = 0; bj < NN; ++bj)
-                        for (int ai = 0; ai < NN; ++ai) {
-                            const R mv = m[nidx(ai, bj, cc)];
-                            const R e2 = mv * mv;
-                            total = total + e2;
-                            if (ai < NN - 1 && bj < NN - 1 && cc < NN - 1) clip1 = clip1 + e2;
-                            if (ai < NN - 2 && bj < NN - 2 && cc < NN - 2) clip2 = clip2 + e2;
-                        }
-                const R e1 = (total - clip1) / total;
-                const R e2 = (clip1 - clip2) / clip1;
-                const R energy = fmax(e1, e2);
-                R al = R(1.0) / (R(1.0) + expneg((R)k.ind_k * (energy - (R)k.ind_T)));
-                if (al < (R)k.alpha_min) al = R(0.0);
-                else if (al > (R)k.one_m_alpha_min) al = R(1.0);
-                s_am[tid] = fmin((R)k.alpha_max, al);
-                int fb = 0;
-                if (learned) {
-                    R rs = R(0.0), ps = R(0.0), rmin = R(1e30), pmin = R(1e30);
-                    for (int n = 0; n < NP; ++n) {
-                        R uu[V];
-    #pragma unroll
-                        for (int v = 0; v < V; ++v) uu[v] = (R)su[(v * EPC + tid) * NP + n];
-                        const R pr = m_pressure(uu, kap, mu0);
-                        rs = rs + uu[0];
-                        ps = ps + pr;
-                        rmin = fmin(rmin, uu[0]);
-                        pmin = fmin(pmin, pr);
-                    }
-                    if (rmin < R(0.1) * (rs / R(64.0)) || pmin < R(0.1) * (ps / R(64.0))) fb = 1;
-                    for (int w = 0; w < 2; ++w) {
-                        const R* mw = scr + (4 + w) * EPC * NP + tid * NP;
-                        R tot = R(0.0), Eo[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
-                        for (int cc = 0; cc < NN; ++cc)
-                            for (int bj = 0; bj < NN; ++bj)
-                                for (int ai = 0; ai < NN; ++ai) {
-                                    const R mv = mw[nidx(ai, bj, cc)];
-                                    const R ee = mv * mv;
-                                    tot = tot + ee;
-                                    const int ord[3] = {ai, bj, cc};
-    #pragma unroll
-                                    for (int d = 0; d < 3; ++d) {
-                                        if (ord[d] == NN - 1) Eo[2 * d] = Eo[2 * d] + ee;
-                                        if (ord[d] == NN - 2) Eo[2 * d + 1] = Eo[2 * d + 1] + ee;
-                                    }
-                                }
-                        for (int i = 0; i < 6; ++i) {
-                            const R f = mlog(Eo[i] / tot + R(1e-12));
-                            feat[tid * 12 + 6 * w + i] = f;
-                            const R x = f / R(10.0) + R(1.0);
-                            if (x < W[MLP_NW + 6 * w + i] || x > W[MLP_NW + 12 + 6 * w + i]) fb = 1;
-                        }
-                    }
-                }
-                s_fb[tid] = fb;
-            }
         }
         __syncthreads();
         if (learned) {
@@ -424,13 +352,12 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
 }  // namespace mhd
 
 // FP32 form: 3 CTAs per SM (168 registers, a few hundred bytes of spills; 2 % faster on B200 than
-// 4 CTAs at 128 registers with twice the spills, and 2 CTAs without spills is 14 % slower);
-// plain FP64: 1 CTA per SM with the full register file.  The conserved state is read per node pair
+// 4 CTAs at 128 registers with twice the spills, and 2 CTAs without spills is 14 % slower).  The conserved state is read per node pair
 // from the FP64 tile: a shared-memory array of per-node FP32 primitives (20 KB more per CTA) made the
 // pair fluxes cheaper but the stage 4 % slower, as the larger carveout left L1 too small for the
 // neighbour traces and register rows.
 template <typename R, bool BLEND, bool RHS_ONLY, bool FAST>
-__global__ void __launch_bounds__(mhd::NT, sizeof(R) == 4 ? NEMO_MHD32_MINB : NEMO_MHD64_MINB) k_stage_mhd(StageArgs a) {
+__global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArgs a) {
     constexpr int MEPC = mhd::EPC, MV = mhd::V;
     using mhd::load_rot;
     using mhd::load_rot_global;
@@ -495,17 +422,18 @@ __global__ void __launch_bounds__(mhd::NT, sizeof(R) == 4 ? NEMO_MHD32_MINB : NE
 #pragma unroll
             for (int i = 0; i < NN; ++i) idx[i] = line_node(d, la, lb, i);
             // ---- surface flux + own-side non-conservative term at both ends
-            // the flux at one end: side 0 the face 2d (neighbour on the left), side 1 the face 2d+1
-            auto side_flux = [&](const int side, R* Fo) {
+            R Fs[2][MV];
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
                 const int f = 2 * d + side;
                 R uo[MV], un[MV], F[MV], G[MV];
-                load_rot(su, el, line_node(d, la, lb, side ? NN - 1 : 0), d, uo);
+                load_rot(su, el, idx[side ? NN - 1 : 0], d, uo);
                 const int32_t ne = a.nbr[e * 6 + f];
                 if (ne <= -2) {  // 2:1 mortar face: flux row (incl. the own-side NC term) of the mortar kernel
                     const double* mf = a.mflux + (int64_t)(-2 - ne) * MV * NF + ab;
 #pragma unroll
-                    for (int v = 0; v < MV; ++v) Fo[v] = (R)mf[v * NF];
-                    return;
+                    for (int v = 0; v < MV; ++v) Fs[side][v] = (R)mf[v * NF];
+                    continue;
                 }
                 if (ne >= 0) {
                     const int nn = line_node(d, la, lb, side ? 0 : NN - 1);
@@ -516,66 +444,15 @@ __global__ void __launch_bounds__(mhd::NT, sizeof(R) == 4 ? NEMO_MHD32_MINB : NE
 #pragma unroll
                     for (int v = 0; v < MV; ++v) un[v] = uo[v];
                 }
-                R uL[MV], uR[MV];
-#pragma unroll
-                for (int v = 0; v < MV; ++v) {
-                    uL[v] = side ? uo[v] : un[v];
-                    uR[v] = side ? un[v] : uo[v];
-                }
-                m_riem<FAST>(a.surface_flux, uL, uR, F, kap, mu0, ch);
-                m_nc_x(uo, uL, uR, G, mu0);
-#pragma unroll
-                for (int v = 0; v < MV; ++v) Fo[v] = F[v] + G[v];
-            };
-            R Fs[2][MV];
-            if constexpr (sizeof(R) == 8) {
-                // plain form: both ends in a rolled loop (one inlined Riemann solver instead of two: 9 %
-                // per stage); the fluxes pass through the thread's subcell slots (free until the
-                // subcell fluxes) into registers.  The FP32 form keeps both ends inlined (its rolled
-                // loop was 0.4 % slower).
-#pragma unroll 1
-                for (int side = 0; side < 2; ++side) {
-                    R Fo[MV];
-                    side_flux(side, Fo);
-#pragma unroll
-                    for (int v = 0; v < MV; ++v) sFh[(side * MV + v) * mhd::NT + tid] = Fo[v];
+                if (side) {
+                    m_riem<FAST>(a.surface_flux, uo, un, F, kap, mu0, ch);
+                    m_nc_x(uo, uo, un, G, mu0);
+                } else {
+                    m_riem<FAST>(a.surface_flux, un, uo, F, kap, mu0, ch);
+                    m_nc_x(uo, un, uo, G, mu0);
                 }
 #pragma unroll
-                for (int side = 0; side < 2; ++side)
-#pragma unroll
-                    for (int v = 0; v < MV; ++v) Fs[side][v] = sFh[(side * MV + v) * mhd::NT + tid];
-            } else {
-#pragma unroll
-                for (int side = 0; side < 2; ++side) {
-                    const int f = 2 * d + side;
-                    R uo[MV], un[MV], F[MV], G[MV];
-                    load_rot(su, el, idx[side ? NN - 1 : 0], d, uo);
-                    const int32_t ne = a.nbr[e * 6 + f];
-                    if (ne <= -2) {  // 2:1 mortar face: flux row (incl. the own-side NC term) of the mortar kernel
-                        const double* mf = a.mflux + (int64_t)(-2 - ne) * MV * NF + ab;
-#pragma unroll
-                        for (int v = 0; v < MV; ++v) Fs[side][v] = (R)mf[v * NF];
-                        continue;
-                    }
-                    if (ne >= 0) {
-                        const int nn = line_node(d, la, lb, side ? 0 : NN - 1);
-                        const int64_t nl = (int64_t)ne - e0;
-                        if (nl >= 0 && nl < nel) load_rot(su, (int)nl, nn, d, un);
-                        else load_rot_global(a.u_in, E, ne, nn, d, un);
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < MV; ++v) un[v] = uo[v];
-                    }
-                    if (side) {
-                        m_riem<FAST>(a.surface_flux, uo, un, F, kap, mu0, ch);
-                        m_nc_x(uo, uo, un, G, mu0);
-                    } else {
-                        m_riem<FAST>(a.surface_flux, un, uo, F, kap, mu0, ch);
-                        m_nc_x(uo, un, uo, G, mu0);
-                    }
-#pragma unroll
-                    for (int v = 0; v < MV; ++v) Fs[side][v] = F[v] + G[v];
-                }
+                for (int v = 0; v < MV; ++v) Fs[side][v] = F[v] + G[v];
             }
             // ---- volume: EC flux + non-conservative term, 6 pairs in the oracle's order
             R t[NN][MV];
@@ -677,13 +554,12 @@ __global__ void __launch_bounds__(mhd::NT, sizeof(R) == 4 ? NEMO_MHD32_MINB : NE
             const int n = nidx(i, la, lb);
             double uu[MV];
             // the node's register values are loaded before any is stored (interleaved, each load
-            // would wait for the previous store); the FP32 form reads them from L2 only (0.7 %
-            // faster; the FP64 form is not)
+            // would wait for the previous store), from L2 only (0.7 % faster)
             double rgv[MV];
 #pragma unroll
             for (int v = 0; v < MV; ++v) {
                 const int64_t g = ((int64_t)v * E + e) * NP + n;
-                rgv[v] = (RHS_ONLY || st == 0) ? 0.0 : (sizeof(R) == 4 ? __ldcg(a.reg + g) : a.reg[g]);
+                rgv[v] = (RHS_ONLY || st == 0) ? 0.0 : __ldcg(a.reg + g);
             }
 #pragma unroll
             for (int v = 0; v < MV; ++v) {
@@ -708,12 +584,9 @@ __global__ void __launch_bounds__(mhd::NT, sizeof(R) == 4 ? NEMO_MHD32_MINB : NE
     if (RHS_ONLY) return;
     __syncthreads();
     if (a.positivity && active && s_bad[el]) {
-        if constexpr (sizeof(R) == 4) {   // FP32 form: the element's 16 threads (a half-warp) together
-            const bool repaired = repair_elem16_mhd<mhd::EPC>(su, el, ab, k);
-            if (!repaired && ab == 0) atomicAdd(&ctrl->nbad, 1ull);
-        } else if (ab == 0) {             // plain form: one thread (register budget of the FP64 kernel)
-            if (!repair_elem_mhd<mhd::EPC>(su, el, k)) atomicAdd(&ctrl->nbad, 1ull);
-        }
+        // the element's 16 threads (a half-warp) together
+        const bool repaired = repair_elem16_mhd<mhd::EPC>(su, el, ab, k);
+        if (!repaired && ab == 0) atomicAdd(&ctrl->nbad, 1ull);
     }
     __syncthreads();
     if (active) {

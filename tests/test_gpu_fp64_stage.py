@@ -76,3 +76,36 @@ def test_quotients_next_to_powers_of_two(base, sf):
     s.upload(u)
     o = orc.Oracle.for_mesh(c, m)
     assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)))
+
+
+def mhd_state(m, seed, mu0):
+    """Smooth periodic GLM-MHD state, every variable its own sinusoid, jumps between some nodes."""
+    u5 = setups.smooth_random(m, seed=seed, kappa=5.0 / 3.0)
+    x, y, z = m.node_coords(setups.LGL4)
+    b = [0.3 + 0.2 * np.sin(2 * np.pi * (x + y)), -0.1 * np.cos(2 * np.pi * z), 0.15 * np.sin(2 * np.pi * (y - z))]
+    psi = 0.02 * np.cos(2 * np.pi * x)
+    b[0][:, 17] += 0.4
+    u = np.concatenate([u5, np.stack(b + [psi])])
+    u[4] += 0.5 / mu0 * (b[0] ** 2 + b[1] ** 2 + b[2] ** 2 + psi ** 2)
+    u[:5, :, 17] *= 1.5
+    u[4, :, 17] += 1.0
+    return np.ascontiguousarray(u)
+
+
+@pytest.mark.parametrize("blend", [False, True])
+@pytest.mark.parametrize("vf,sf,mu0", [(abi.VOLFLUX_EC_MHD, abi.SURFFLUX_HLLD, 1.0), (abi.VOLFLUX_CENTRAL, abi.SURFFLUX_HLLD, 1.0),
+                                       (abi.VOLFLUX_EC_MHD, abi.SURFFLUX_RUSANOV, 1.3)])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_mhd_steps_bit_exact(name, vf, sf, mu0, blend):
+    m = MESHES[name]()
+    u = mhd_state(m, 5, mu0)
+    c = abi.default_cfg(eqn=abi.EQN_MHD, n_vars=9, volume_flux=vf, surface_flux=sf, kappa=5.0 / 3.0, mu0=mu0, positivity=1,
+                        indicator=abi.IND_MODAL if blend else abi.IND_NONE, glm_ch=0.7, glm_alpha=0.3)
+    s = Solver(c, m)
+    o = orc.Oracle.for_mesh(c, m)
+    s.upload(u)
+    assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)) if blend else o.rhs(u))
+    t, n = s.run(nsteps=3)
+    ref, tr, nr, _ = o.run(u, nsteps=3)
+    assert t == tr and n == nr
+    assert np.array_equal(s.download(), ref)
