@@ -287,24 +287,23 @@ __device__ __forceinline__ void epilogue32(const StageArgs& a, const double* su,
     __shared__ double s_dt[EPC], s_lm[EPC];
     __shared__ int s_gr[EPC];
     if (threadIdx.x < EPC) s_fb[threadIdx.x] = 0;
+    // the thread reads nodes ab + 16 i of the FP64 state (no bank conflicts) and hands rho and p on
+    // through the scratch to the threads of their x-lines
     float qr[NN], qp[NN];
     float lx = 0.f, ly = 0.f, lz = 0.f;
-#pragma unroll
-    for (int i = 0; i < NN; ++i) {
-        qr[i] = 1.f;
-        qp[i] = 1.f;
-    }
+    float* xr = scratch + 6 * EPC * SP;   // [EPC][64] rho, then p
+    float* xp = scratch + 7 * EPC * SP;
     if (active) {
 #pragma unroll
         for (int i = 0; i < NN; ++i) {
-            const int n = nidx(i, la, lb);
+            const int n = ab + 16 * i;
             const double r = su[(0 * EPC + el) * NP + n];
             const double mx = su[(1 * EPC + el) * NP + n], my = su[(2 * EPC + el) * NP + n];
             const double mz = su[(3 * EPC + el) * NP + n], en = su[(4 * EPC + el) * NP + n];
             const double ir = rcp64(r);
             const double prd = k.km1 * (en - 0.5 * ir * (mx * mx + my * my + mz * mz));
-            qr[i] = (float)r;
-            qp[i] = (float)prd;
+            xr[el * SP + n] = (float)r;
+            xp[el * SP + n] = (float)prd;
             if (need_lam) {
                 const float c = sqrtf((float)(k.kappa * prd * ir));
                 lx = fmaxf(lx, fabsf((float)(mx * ir)) + c);
@@ -312,6 +311,12 @@ __device__ __forceinline__ void epilogue32(const StageArgs& a, const double* su,
                 lz = fmaxf(lz, fabsf((float)(mz * ir)) + c);
             }
         }
+    }
+    __syncwarp();   // the element's 16 threads share one warp
+#pragma unroll
+    for (int i = 0; i < NN; ++i) {
+        qr[i] = active ? xr[el * SP + nidx(i, la, lb)] : 1.f;
+        qp[i] = active ? xp[el * SP + nidx(i, la, lb)] : 1.f;
     }
     if (a.alpha_out) {
         const bool learned = learned_form;
@@ -646,11 +651,12 @@ __device__ __forceinline__ void tile32(const StageArgs& a, const Smem32& S, int6
     }
     auto SQ = [&](int q, int elx, int n) -> float& { return sq[(q * EPC + elx) * SP + n]; };
 
-    // per-node primitives of the thread's x-line nodes: recovered in FP64, stored in FP32
+    // per-node primitives: recovered in FP64, stored in FP32; a thread takes nodes ab + 16 q, so that
+    // the FP64 rows are read without bank conflicts (its x-line nodes, stride 4, conflict four ways)
     if (active) {
 #pragma unroll
         for (int i = 0; i < NN; ++i) {
-            const int n = nidx(i, la, lb);
+            const int n = ab + 16 * i;
             const double r = su[(0 * EPC + el) * NP + n];
             const double mx = su[(1 * EPC + el) * NP + n], my = su[(2 * EPC + el) * NP + n];
             const double mz = su[(3 * EPC + el) * NP + n], en = su[(4 * EPC + el) * NP + n];
@@ -729,7 +735,7 @@ __device__ __forceinline__ void tile32(const StageArgs& a, const Smem32& S, int6
                         const double m1 = __ldcg(g + ((int64_t)(1 + c1) * E + ne) * NP + nn);
                         const double m2 = __ldcg(g + ((int64_t)(1 + c2) * E + ne) * NP + nn);
                         const double en = __ldcg(g + ((int64_t)4 * E + ne) * NP + nn);
-                        const double ir = 1.0 / r;
+                        const double ir = quot64(1.0, rcp64r(r));   // 1/r, the same bits without a branch
                         const double v0 = m0 * ir, v1 = m1 * ir, v2 = m2 * ir;
                         qn.rho = (float)r;
                         qn.vn = (float)v0;
