@@ -352,7 +352,9 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
 }  // namespace mhd
 
 // FP32 form: 3 CTAs per SM (168 registers, a few hundred bytes of spills; 2 % faster on B200 than
-// 4 CTAs at 128 registers with twice the spills, and 2 CTAs without spills is 14 % slower).  The conserved state is read per node pair
+// 4 CTAs at 128 registers with twice the spills, and 2 CTAs without spills is 14 % slower).  The update takes
+// nodes ab + 16 q of its element, coalesced rows of the register and the state (the x-line nodes, 32 bytes
+// apart, moved four sectors for one: 401 -> 336 us per stage at Orszag-Tang 32^3).  The conserved state is read per node pair
 // from the FP64 tile: a shared-memory array of per-node FP32 primitives (20 KB more per CTA) made the
 // pair fluxes cheaper but the stage 4 % slower, as the larger carveout left L1 too small for the
 // neighbour traces and register rows.
@@ -551,7 +553,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
         bool ok = true;
 #pragma unroll
         for (int i = 0; i < NN; ++i) {
-            const int n = nidx(i, la, lb);
+            const int n = ab + 16 * i;   // rows: coalesced in global memory, no bank conflicts
             double uu[MV];
             // the node's register values are loaded before any is stored (interleaved, each load
             // would wait for the previous store), from L2 only (0.7 % faster)
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
         for (int v = 0; v < MV; ++v)
 #pragma unroll
             for (int i = 0; i < NN; ++i) {
-                const int n = nidx(i, la, lb);
+                const int n = ab + 16 * i;
                 a.u_out[((int64_t)v * E + e) * NP + n] = su[(v * MEPC + el) * NP + n];
             }
     }
