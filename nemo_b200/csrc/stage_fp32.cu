@@ -1085,10 +1085,9 @@ cudaError_t setup_stage_euler32(const OpConsts& ops) {
 namespace nemo {
 #undef NEMO_MHD_OPS
 
-// state, rhs rows and the subcell interface fluxes of each thread's line
+// the FP64 tile (and what takes its place) and its FP32 copy
 int stage_smem_bytes_mhd32() {
-    return mhd::V * mhd::EPC * (NP * (int)sizeof(double) + mhd::SPM * (int)sizeof(float)) +
-           (NN - 1) * mhd::V * mhd::NT * (int)sizeof(float);
+    return mhd::V * mhd::EPC * (NP * (int)sizeof(double) + mhd::SPM * (int)sizeof(float));
 }
 
 cudaError_t setup_stage_mhd32() {

@@ -24,7 +24,9 @@ namespace nemo {
 namespace mhd {
 
 // Tile shape: elements per CTA (16 threads each) and the resident CTAs per SM asked of the register allocator
+#ifndef NEMO_MHD32_MINB
 #define NEMO_MHD32_MINB 3
+#endif
 constexpr int EPC = 8;
 constexpr int NT = 16 * EPC;
 constexpr int V = 9;
@@ -50,7 +52,7 @@ __device__ __forceinline__ bool mbar_wait_m(uint64_t* bar, unsigned phase) {
 
 // The tile's bulk copy: issue (barrier set-up, thread 0 starts the copies), then, after other work,
 // the wait.
-__device__ __forceinline__ void tile_issue_m(double* su, const double* __restrict__ u, int64_t E, int64_t e0, int nel,
+__device__ __forceinline__ void tile_issue_m(double* su, const double* __restrict__ u, const double* __restrict__ reg, int64_t E, int64_t e0, int nel,
                                              uint64_t* bar) {
     if (threadIdx.x == 0) {
         const unsigned b = su32(bar);
@@ -69,6 +71,10 @@ __device__ __forceinline__ void tile_issue_m(double* su, const double* __restric
                     su32(su + v * EPC * NP)),
                 "l"(u + ((int64_t)v * E + e0) * NP), "r"(bytes), "r"(b)
                 : "memory");
+        if (reg)   // the register rows, needed at the end
+            for (int v = 0; v < V; ++v)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reg + ((int64_t)v * E + e0) * NP), "r"(bytes)
+                             : "memory");
     }
 }
 
@@ -81,16 +87,17 @@ __device__ __forceinline__ bool tile_wait_m(uint64_t* bar, Control* ctrl) {
     return ok;
 }
 
-// rotated state of node n of element el (momentum and field cyclically into direction d)
+// rotated state of node n of element el (momentum and field cyclically into direction d), from the FP32
+// copy of the tile [9][EPC][SPM]
 template <typename R>
-__device__ __forceinline__ void load_rot(const double* su, int el, int n, int d, R* r) {
-    r[0] = (R)su[(0 * EPC + el) * NP + n];
-    r[4] = (R)su[(4 * EPC + el) * NP + n];
-    r[8] = (R)su[(8 * EPC + el) * NP + n];
+__device__ __forceinline__ void load_rot(const R* sq, int el, int n, int d, R* r) {
+    r[0] = sq[(0 * EPC + el) * SPM + n];
+    r[4] = sq[(4 * EPC + el) * SPM + n];
+    r[8] = sq[(8 * EPC + el) * SPM + n];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        r[1 + c] = (R)su[((1 + (d + c) % 3) * EPC + el) * NP + n];
-        r[5 + c] = (R)su[((5 + (d + c) % 3) * EPC + el) * NP + n];
+        r[1 + c] = sq[((1 + (d + c) % 3) * EPC + el) * SPM + n];
+        r[5 + c] = sq[((5 + (d + c) % 3) * EPC + el) * SPM + n];
     }
 }
 
@@ -365,9 +372,14 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
     using mhd::load_rot_global;
     using mhd::unrot;
     extern __shared__ __align__(128) double smem_m[];
+    // the FP64 tile is turned into an FP32 copy once; its place then holds the rhs terms and the subcell
+    // fluxes, and in the end the new FP64 state
     double* su = smem_m;                                    // [9][MEPC][64] FP64 state
-    R* sR = reinterpret_cast<R*>(su + MV * MEPC * NP);        // [9][MEPC][64] rhs terms
-    R* sFh = sR + MV * MEPC * mhd::SPM;                        // [NN-1][9][NT] subcell interface fluxes
+    R* sR = reinterpret_cast<R*>(su);                       // [9][MEPC][64] rhs terms
+    R* sFh = sR + MV * MEPC * mhd::SPM;                     // [NN-1][9][NT] subcell interface fluxes
+    R* sq = reinterpret_cast<R*>(su + MV * MEPC * NP);      // [9][MEPC][64] FP32 state, then epilogue scratch
+    static_assert(MV * MEPC * NP * 2 >= MV * MEPC * mhd::SPM + (NN - 1) * MV * mhd::NT, "rhs and subcell fluxes fit");
+    static_assert(MV * MEPC * mhd::SPM >= 6 * MEPC * NP, "epilogue scratch fits");
     __shared__ uint64_t bar;
     __shared__ R s_alpha[MEPC];
     __shared__ int s_bad[MEPC];
@@ -385,7 +397,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
     const R ch = (R)ctrl->glm_ch;
 
     // the tile's bulk copy first, so that it is in flight while the blending coefficients are read
-    mhd::tile_issue_m(su, a.u_in, E, e0, nel, &bar);
+    mhd::tile_issue_m(su, a.u_in, RHS_ONLY || a.prep_only || a.stage == 0 ? nullptr : a.reg, E, e0, nel, &bar);
     // the first thread of each element reads its blending coefficient; the element's 16 threads
     // share a warp, so a warp sync makes it visible (no CTA barrier: the loads overlap the bulk copy)
     if ((tid & 15) == 0) {
@@ -411,13 +423,21 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
     if (!mhd::tile_wait_m(&bar, ctrl)) return;
     if (a.prep_only) {
         __syncthreads();
-        mhd::epilogue_mhd<R>(a, su, sR, s_lam, &s_vmax, nel, e0, tid, k);
+        mhd::epilogue_mhd<R>(a, su, sq, s_lam, &s_vmax, nel, e0, tid, k);
         return;
     }
 
     const int el = tid >> 4, ab = tid & 15, la = ab & 3, lb = ab >> 2;
     const bool active = el < nel;
     const int64_t e = e0 + el;
+    if (active) {
+#pragma unroll
+        for (int i = 0; i < NN; ++i)
+#pragma unroll
+            for (int v = 0; v < MV; ++v)
+                sq[(v * MEPC + el) * mhd::SPM + ab + 16 * i] = (R)su[(v * MEPC + el) * NP + ab + 16 * i];
+    }
+    __syncthreads();   // the FP32 copy complete, the FP64 tile free
     for (int d = 0; d < 3; ++d) {
         if (active) {
             int idx[NN];
@@ -429,7 +449,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
             for (int side = 0; side < 2; ++side) {
                 const int f = 2 * d + side;
                 R uo[MV], un[MV], F[MV], G[MV];
-                load_rot(su, el, idx[side ? NN - 1 : 0], d, uo);
+                load_rot(sq, el, idx[side ? NN - 1 : 0], d, uo);
                 const int32_t ne = a.nbr[e * 6 + f];
                 if (ne <= -2) {  // 2:1 mortar face: flux row (incl. the own-side NC term) of the mortar kernel
                     const double* mf = a.mflux + (int64_t)(-2 - ne) * MV * NF + ab;
@@ -440,7 +460,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
                 if (ne >= 0) {
                     const int nn = line_node(d, la, lb, side ? 0 : NN - 1);
                     const int64_t nl = (int64_t)ne - e0;
-                    if (nl >= 0 && nl < nel) load_rot(su, (int)nl, nn, d, un);
+                    if (nl >= 0 && nl < nel) load_rot(sq, (int)nl, nn, d, un);
                     else load_rot_global(a.u_in, E, ne, nn, d, un);
                 } else {
 #pragma unroll
@@ -467,8 +487,8 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
 #pragma unroll
                 for (int m = i + 1; m < NN; ++m) {
                     R ui[MV], um[MV], F[MV], Gi[MV], Gm[MV];
-                    load_rot(su, el, idx[i], d, ui);
-                    load_rot(su, el, idx[m], d, um);
+                    load_rot(sq, el, idx[i], d, ui);
+                    load_rot(sq, el, idx[m], d, um);
                     if (!FAST && a.volume_flux == NEMO_VOLFLUX_CENTRAL) m_central_x(ui, um, F, kap, mu0, ch);
                     else m_ec_x(ui, um, F, kap, mu0, ch);
                     m_nc_x(ui, ui, um, Gi, mu0);
@@ -495,8 +515,8 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
 #pragma unroll 1
                     for (int q = 0; q < NN - 1; ++q) {
                         R uq[MV], ur[MV], Fq[MV];
-                        load_rot(su, el, line_node(d, la, lb, q), d, uq);
-                        load_rot(su, el, line_node(d, la, lb, q + 1), d, ur);
+                        load_rot(sq, el, line_node(d, la, lb, q), d, uq);
+                        load_rot(sq, el, line_node(d, la, lb, q + 1), d, ur);
                         m_riem<FAST>(a.surface_flux, uq, ur, Fq, kap, mu0, ch);
 #pragma unroll
                         for (int v = 0; v < MV; ++v) sFh[(q * MV + v) * mhd::NT + tid] = Fq[v];
@@ -504,10 +524,10 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
 #pragma unroll
                     for (int i = 0; i < NN; ++i) {
                         R ui[MV], FR[MV], FL[MV], G[MV];
-                        load_rot(su, el, idx[i], d, ui);
+                        load_rot(sq, el, idx[i], d, ui);
                         if (i > 0) {
                             R ul[MV];
-                            load_rot(su, el, idx[i - 1], d, ul);
+                            load_rot(sq, el, idx[i - 1], d, ul);
                             m_nc_x(ui, ul, ui, G, mu0);
 #pragma unroll
                             for (int v = 0; v < MV; ++v) FL[v] = sFh[((i - 1) * MV + v) * mhd::NT + tid] + G[v];
@@ -517,7 +537,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
                         }
                         if (i < NN - 1) {
                             R ur[MV];
-                            load_rot(su, el, idx[i + 1], d, ur);
+                            load_rot(sq, el, idx[i + 1], d, ur);
                             m_nc_x(ui, ui, ur, G, mu0);
 #pragma unroll
                             for (int v = 0; v < MV; ++v) FR[v] = sFh[(i * MV + v) * mhd::NT + tid] + G[v];
@@ -549,25 +569,26 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
     const double A = rk_a(st);
     const double cdt = rk_c(st) * ctrl->dt[0];
     const double galpha = ctrl->glm_alpha;
+    double un[NN][MV];   // the new state of nodes ab + 16 i
     if (active) {
         bool ok = true;
 #pragma unroll
         for (int i = 0; i < NN; ++i) {
             const int n = ab + 16 * i;   // rows: coalesced in global memory, no bank conflicts
-            double uu[MV];
-            // the node's register values are loaded before any is stored (interleaved, each load
-            // would wait for the previous store), from L2 only (0.7 % faster)
+            // the node's register and state values (read again from L2: shared memory holds the rhs terms in
+            // the tile's place) are loaded before any is stored (interleaved, each load would wait for the
+            // previous store), from L2 only (0.7 % faster)
             double rgv[MV];
 #pragma unroll
             for (int v = 0; v < MV; ++v) {
                 const int64_t g = ((int64_t)v * E + e) * NP + n;
                 rgv[v] = (RHS_ONLY || st == 0) ? 0.0 : __ldcg(a.reg + g);
+                un[i][v] = RHS_ONLY && v != 8 ? 0.0 : __ldcg(a.u_in + g);
             }
 #pragma unroll
             for (int v = 0; v < MV; ++v) {
-                const int s = (v * MEPC + el) * NP + n;
                 double rhs = -(double)sR[(v * MEPC + el) * mhd::SPM + n];
-                if (v == 8) rhs = rhs - galpha * su[s];
+                if (v == 8) rhs = rhs - galpha * un[i][v];
                 const int64_t g = ((int64_t)v * E + e) * NP + n;
                 if (RHS_ONLY) {
                     a.rhs_out[g] = rhs;
@@ -575,15 +596,21 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
                     const double rg = rgv[v];
                     const double r2 = st == 0 ? rhs : A * rg + rhs;
                     a.reg[g] = r2;
-                    su[s] = su[s] + cdt * r2;
+                    un[i][v] = un[i][v] + cdt * r2;
                 }
-                uu[v] = su[s];
             }
-            if (!RHS_ONLY && a.positivity) ok = ok && m_isvalid(uu, k.kappa, k.mu0);
+            if (!RHS_ONLY && a.positivity) ok = ok && m_isvalid(un[i], k.kappa, k.mu0);
         }
         if (!ok) s_bad[el] = 1;
     }
     if (RHS_ONLY) return;
+    __syncthreads();   // every element's rhs terms are used up
+    if (active) {
+#pragma unroll
+        for (int i = 0; i < NN; ++i)
+#pragma unroll
+            for (int v = 0; v < MV; ++v) su[(v * MEPC + el) * NP + ab + 16 * i] = un[i][v];
+    }
     __syncthreads();
     if (a.positivity && active && s_bad[el]) {
         // the element's 16 threads (a half-warp) together
@@ -605,7 +632,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
         ctrl->steps += 1;
     }
     __syncthreads();
-    mhd::epilogue_mhd<R>(a, su, sR, s_lam, &s_vmax, nel, e0, tid, k);
+    mhd::epilogue_mhd<R>(a, su, sq, s_lam, &s_vmax, nel, e0, tid, k);
 }
 
 }  // namespace nemo
