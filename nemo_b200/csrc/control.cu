@@ -26,6 +26,8 @@ __global__ void k_ctrl_set_dt(Control* c, double dt) {
 // step's last stage (or by a prepare launch): dt = factor * min(delta/lambda), clamped to t_end.
 __global__ void k_ctrl_step(Control* c) {
     __shared__ int s_live;
+    dep_sync();
+    dep_launch();
     if (threadIdx.x == 0) {
         s_live = 0;
         if (c->mhd) {  // GLM cleaning speed and damping of this step (kernel_timestep_mod.f90:338-344)
@@ -173,8 +175,7 @@ cudaError_t launch_ctrl_set_dt(Control* c, double dt, cudaStream_t s) {
 }
 
 cudaError_t launch_ctrl_step(Control* c, cudaStream_t s) {
-    k_ctrl_step<<<1, 256, 0, s>>>(c);
-    return cudaGetLastError();
+    return launch_dep(k_ctrl_step, 1, 256, 0, s, c);
 }
 
 cudaError_t launch_aos_to_soa(const double* aos, double* soa, int64_t E, int nv, cudaStream_t s) {

@@ -906,6 +906,7 @@ __device__ __forceinline__ void tile32(const StageArgs& a, const Smem32& S, int6
         ctrl->steps += 1;
     }
 
+    if (!PERSIST) dep_launch();
     epilogue32<EPC, FAST>(a, su, sq, s_w, el, ab, la, lb, active, e, k);
     if (tid == 0) tile_store_wait32();
 }
@@ -917,11 +918,12 @@ __global__ void __launch_bounds__(EPC * TPE, 32 / EPC) k_stage_euler32(StageArgs
     __shared__ uint64_t bar[1];
     __shared__ float s_alpha[EPC];
     __shared__ int s_bad[EPC];
+    mbar_init32(bar);
+    dep_sync();
     if (!RHS_ONLY && !a.prep_only && a.ctrl->done) return;
     // the learned indicator's weights are read through L1 by the epilogue (a CTA handles one tile:
     // a shared-memory copy of the 6 KB per CTA would cost more L2 reads than it saves)
     const Smem32 S = smem32<EPC>(smem, bar, s_alpha, s_bad, a.mlp32t);
-    mbar_init32(bar);
     tile32<EPC, BLEND, RHS_ONLY, false, FAST>(a, S, (int64_t)blockIdx.x, 0u, 0u);
 }
 
@@ -993,16 +995,15 @@ static cudaError_t launch32(const StageArgs& a, bool blend, bool rhs_only, cudaS
     if (grid <= 0) return cudaSuccess;
     const int smem = stage_smem_bytes32(EPC), nt = EPC * TPE;
     if (rhs_only) {
-        if (blend) k_stage_euler32<EPC, true, true, false><<<grid, nt, smem, s>>>(a);
-        else k_stage_euler32<EPC, false, true, false><<<grid, nt, smem, s>>>(a);
-    } else if (fast_form(a)) {
-        if (blend) k_stage_euler32<EPC, true, false, true><<<grid, nt, smem, s>>>(a);
-        else k_stage_euler32<EPC, false, false, true><<<grid, nt, smem, s>>>(a);
-    } else {
-        if (blend) k_stage_euler32<EPC, true, false, false><<<grid, nt, smem, s>>>(a);
-        else k_stage_euler32<EPC, false, false, false><<<grid, nt, smem, s>>>(a);
+        if (blend) return launch_dep(k_stage_euler32<EPC, true, true, false>, grid, nt, smem, s, a);
+        return launch_dep(k_stage_euler32<EPC, false, true, false>, grid, nt, smem, s, a);
     }
-    return cudaGetLastError();
+    if (fast_form(a)) {
+        if (blend) return launch_dep(k_stage_euler32<EPC, true, false, true>, grid, nt, smem, s, a);
+        return launch_dep(k_stage_euler32<EPC, false, false, true>, grid, nt, smem, s, a);
+    }
+    if (blend) return launch_dep(k_stage_euler32<EPC, true, false, false>, grid, nt, smem, s, a);
+    return launch_dep(k_stage_euler32<EPC, false, false, false>, grid, nt, smem, s, a);
 }
 
 cudaError_t launch_stage_euler32(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s, int epc) {
@@ -1109,16 +1110,15 @@ cudaError_t launch_stage_mhd32(const StageArgs& a, bool blend, bool rhs_only, cu
     // the specialised kernel for HLLD faces and the EC pair flux, the general one for the rest
     const bool fast = a.surface_flux == NEMO_SURFFLUX_HLLD && a.volume_flux == NEMO_VOLFLUX_EC_MHD;
     if (rhs_only) {
-        if (blend) k_stage_mhd<float, true, true, false><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<float, false, true, false><<<grid, mhd::NT, smem, s>>>(a);
-    } else if (fast) {
-        if (blend) k_stage_mhd<float, true, false, true><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<float, false, false, true><<<grid, mhd::NT, smem, s>>>(a);
-    } else {
-        if (blend) k_stage_mhd<float, true, false, false><<<grid, mhd::NT, smem, s>>>(a);
-        else k_stage_mhd<float, false, false, false><<<grid, mhd::NT, smem, s>>>(a);
+        if (blend) return launch_dep(k_stage_mhd<float, true, true, false>, grid, mhd::NT, smem, s, a);
+        return launch_dep(k_stage_mhd<float, false, true, false>, grid, mhd::NT, smem, s, a);
     }
-    return cudaGetLastError();
+    if (fast) {
+        if (blend) return launch_dep(k_stage_mhd<float, true, false, true>, grid, mhd::NT, smem, s, a);
+        return launch_dep(k_stage_mhd<float, false, false, true>, grid, mhd::NT, smem, s, a);
+    }
+    if (blend) return launch_dep(k_stage_mhd<float, true, false, false>, grid, mhd::NT, smem, s, a);
+    return launch_dep(k_stage_mhd<float, false, false, false>, grid, mhd::NT, smem, s, a);
 }
 
 }  // namespace nemo

@@ -281,8 +281,6 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
 
     const OpConsts& k = c_ops64;
     Control* ctrl = a.ctrl;
-    if (!RHS_ONLY && ctrl->done) return;
-
     const int n = threadIdx.x, lane = n & 31, w = n >> 5;
     const int64_t E = a.E;
     const int64_t e = a.E_begin + blockIdx.x;
@@ -291,6 +289,10 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
         s_vi[n] = k.Vinv[n];
         if (n < NN) s_winv[n] = k.winv[n];
     }
+    // faces p of the neighbour traces this thread fetches, p = n and (warp 0) n + 64
+    const int32_t nes[2] = {__ldg(a.nbr + e * 6 + (n >> 4)), n < 6 * NF - TPE ? __ldg(a.nbr + e * 6 + 4 + (n >> 4)) : -1};
+    dep_sync();
+    if (!RHS_ONLY && ctrl->done) return;
     double* const su = smem + O_SU;
     double* const sp = smem + O_SP;
     double* const tr = smem + O_TR;
@@ -313,9 +315,11 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
     }
 
     // neighbour traces (or mortar flux rows) of the 96 face nodes, asynchronously
-    for (int p = n; p < 6 * NF; p += TPE) {
-        const int f = p >> 4, ab = p & 15;
-        const int32_t ne = __ldg(a.nbr + e * 6 + f);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int p = n + r * TPE, f = p >> 4, ab = p & 15;
+        if (p >= 6 * NF) break;
+        const int32_t ne = nes[r];
         if (ab == 0) s_nbr[f] = ne;
         if (ne >= 0) {
             const double* g = a.u_in + (int64_t)ne * NP + line_node(f >> 1, ab & 3, ab >> 2, (f & 1) ? 0 : NN - 1);
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
         for (int g = 0; g < ctrl->ngroups; ++g) ctrl->t[g] = ctrl->t[g] + ctrl->dt[g];
         ctrl->steps += 1;
     }
-
+    dep_launch();
     epilogue();
 }
 
@@ -554,16 +558,15 @@ cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool rhs_only, 
     // the specialised kernel for HLLC faces and Chandrashekar pairs, the general one for the rest
     const bool fast = a.surface_flux == NEMO_SURFFLUX_HLLC && a.volume_flux == NEMO_VOLFLUX_CHANDRASHEKAR;
     if (rhs_only) {
-        if (blend) k_stage_euler64<true, true, false><<<grid, TPE, smem, s>>>(a);
-        else k_stage_euler64<false, true, false><<<grid, TPE, smem, s>>>(a);
-    } else if (fast) {
-        if (blend) k_stage_euler64<true, false, true><<<grid, TPE, smem, s>>>(a);
-        else k_stage_euler64<false, false, true><<<grid, TPE, smem, s>>>(a);
-    } else {
-        if (blend) k_stage_euler64<true, false, false><<<grid, TPE, smem, s>>>(a);
-        else k_stage_euler64<false, false, false><<<grid, TPE, smem, s>>>(a);
+        if (blend) return launch_dep(k_stage_euler64<true, true, false>, grid, TPE, smem, s, a);
+        return launch_dep(k_stage_euler64<false, true, false>, grid, TPE, smem, s, a);
     }
-    return cudaGetLastError();
+    if (fast) {
+        if (blend) return launch_dep(k_stage_euler64<true, false, true>, grid, TPE, smem, s, a);
+        return launch_dep(k_stage_euler64<false, false, true>, grid, TPE, smem, s, a);
+    }
+    if (blend) return launch_dep(k_stage_euler64<true, false, false>, grid, TPE, smem, s, a);
+    return launch_dep(k_stage_euler64<false, false, false>, grid, TPE, smem, s, a);
 }
 
 // The largest carveout: twelve elements take 220 KB of an SM's shared memory, and the kernel reads

@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
 
     const OpConsts& k = NEMO_MHD_OPS;
     Control* ctrl = a.ctrl;
+    dep_sync();
     if (!RHS_ONLY && !a.prep_only && ctrl->done) return;
     const int tid = threadIdx.x;
     const int64_t E = a.E;
@@ -631,6 +632,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
         for (int g = 0; g < ctrl->ngroups; ++g) ctrl->t[g] = ctrl->t[g] + ctrl->dt[g];
         ctrl->steps += 1;
     }
+    dep_launch();
     __syncthreads();
     mhd::epilogue_mhd<R>(a, su, sq, s_lam, &s_vmax, nel, e0, tid, k);
 }
