@@ -109,3 +109,18 @@ def test_mhd_steps_bit_exact(name, vf, sf, mu0, blend):
     ref, tr, nr, _ = o.run(u, nsteps=3)
     assert t == tr and n == nr
     assert np.array_equal(s.download(), ref)
+
+
+@pytest.mark.parametrize("box", [(1, 1, 1), (3, 21, 1), (4, 4, 4), (5, 13, 1), (11, 31, 3), (16, 8, 8), (5, 5, 41), (3, 683, 1)])
+def test_totals_at_chunk_edges(box):
+    """Conserved totals around the element blocks (64) and the summation chunks (1024): 1, 63, 64, 65, 1023, 1024,
+    1025 and 2049 elements, in the oracle's serial order bit for bit, Euler and GLM-MHD."""
+    m = mesh.brick(*box)
+    for mhd in (False, True):
+        u = mhd_state(m, 2, 1.0) if mhd else setups.smooth_random(m, seed=2)
+        c = abi.default_cfg(eqn=abi.EQN_MHD, n_vars=9, volume_flux=abi.VOLFLUX_EC_MHD, surface_flux=abi.SURFFLUX_HLLD) if mhd \
+            else abi.default_cfg()
+        s = Solver(c, m)
+        s.upload(u)
+        assert np.array_equal(s.totals(), orc.Oracle.for_mesh(c, m).totals(u)[: u.shape[0]])
+        s.finalize()
