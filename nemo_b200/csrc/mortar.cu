@@ -10,7 +10,7 @@ __constant__ OpConsts c_opsm;
 
 template <bool MHD>
 __global__ void __launch_bounds__(128) k_mortar(MortarArgs a) {
-    __shared__ double scratch[mortar::SCRATCH_DOUBLES];
+    __shared__ double scratch[mortar::scratch_doubles(MHD ? 9 : 5)];
     dep_sync();
     if (a.skip_if_done && a.ctrl->done) return;
     mortar::mortar_pair<MHD>(a, (int64_t)blockIdx.x, scratch, c_opsm);

@@ -14,13 +14,16 @@
 
 #include "euler_fp64.cuh"
 #include "kernels.h"
-#include "mhd_phys.cuh"
+#include "mhd_fp64.cuh"
 
 namespace nemo {
 namespace mortar {
 
 constexpr int MPB = 2;          // mortars per 128-thread task
-constexpr int SCRATCH_DOUBLES = MPB * 9 * NF + MPB * 4 * 9 * NF;
+// per mortar: coarse trace [V][16], half-prolonged trace [V][32], later half-projected fluxes [V][64], and the
+// sub-face fluxes [4][V][16]; once per task the two pairs of 1D matrices
+constexpr int scratch_doubles(int V) { return MPB * (V * NF + V * 64 + 4 * V * NF) + 4 * NN * NN; }
+constexpr int SCRATCH_DOUBLES = scratch_doubles(9);
 
 // LGL-weighted mean of a coarse face trace held as [V][NF] (out of line: taken only on a shock)
 static __device__ __noinline__ void face_mean(const double* uc, int V, double* out, const OpConsts& k) {
@@ -36,7 +39,10 @@ template <bool MHD>
 __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, double* scratch, const OpConsts& k) {
     constexpr int V = MHD ? 9 : 5;
     auto s_uc = reinterpret_cast<double (*)[V][NF]>(scratch);                       // [MPB][V][NF]
-    auto s_fs = reinterpret_cast<double (*)[4][V][NF]>(scratch + MPB * V * NF);      // [MPB][4][V][NF]
+    auto s_in = reinterpret_cast<double (*)[V][64]>(scratch + MPB * V * NF);         // [MPB][V][64]
+    auto s_fs = reinterpret_cast<double (*)[4][V][NF]>(scratch + MPB * V * (NF + 64));   // [MPB][4][V][NF]
+    double* s_pro = scratch + MPB * V * (NF + 64 + 4 * NF);                          // [2][16], then prj [2][16]
+    double* s_prj = s_pro + 2 * NN * NN;
     const int ml = threadIdx.x >> 6, r = threadIdx.x & 63;
     const int64_t m = pair * MPB + ml;
     const bool act = m < a.nm;
@@ -45,28 +51,41 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
     const int64_t qc = t[0];
     const int fc = t[1], ff = fc ^ 1, d = fc >> 1;
     const bool coarse_left = (fc & 1) != 0;
+    const int kq = r >> 4, i = r & 3, j = (r >> 2) & 3;
+    const int s = kq & 1, tt = kq >> 1;
+    double up[V], uf[V];
+    if (threadIdx.x < 4 * NN * NN)   // the matrices are indexed per thread: shared, not constant memory
+        s_pro[threadIdx.x] = threadIdx.x < 2 * NN * NN ? k.pro[threadIdx.x >> 4][threadIdx.x & 15]
+                                                       : k.prj[(threadIdx.x >> 4) & 1][threadIdx.x & 15];
     if (act && r < NF) {
         const int n = line_node(d, r & 3, r >> 2, (fc & 1) ? NN - 1 : 0);
 #pragma unroll
         for (int v = 0; v < V; ++v) s_uc[ml][v][r] = a.u_in[((int64_t)v * E + qc) * NP + n];
     }
-    __syncthreads();
-    const int kq = r >> 4, i = r & 3, j = (r >> 2) & 3;
-    const int s = kq & 1, tt = kq >> 1;
     if (act) {
         const int64_t qf = t[2 + kq];
         const int nf = line_node(d, i, j, (ff & 1) ? NN - 1 : 0);
-        double up[V], uf[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) uf[v] = a.u_in[((int64_t)v * E + qf) * NP + nf];
+    }
+    __syncthreads();
+    // prolongation, one axis at a time: the first axis of a row is shared by the four nodes and two sub-faces
+    // along the second
+    if (act)
+        for (int p = r; p < 32 * V; p += 64) {
+            const int v = p >> 5, row = p & 31, bb = row & 3;   // row = (half, node i, bb)
+            double in = 0.0;
+#pragma unroll
+            for (int aa = 0; aa < NN; ++aa) in = in + s_pro[(row >> 2) * NN + aa] * s_uc[ml][v][aa + NN * bb];
+            s_in[ml][v][row] = in;
+        }
+    __syncthreads();
+    if (act) {
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             double acc = 0.0;
 #pragma unroll
-            for (int bb = 0; bb < NN; ++bb) {
-                double in = 0.0;
-#pragma unroll
-                for (int aa = 0; aa < NN; ++aa) in = in + k.pro[s][i * NN + aa] * s_uc[ml][v][aa + NN * bb];
-                acc = acc + k.pro[tt][j * NN + bb] * in;
-            }
+            for (int bb = 0; bb < NN; ++bb) acc = acc + s_pro[tt * NN * NN + j * NN + bb] * s_in[ml][v][s * NF + i * NN + bb];
             up[v] = acc;
         }
         // a sub-face (16 lanes of this warp; act is warp-uniform) whose prolonged trace has an
@@ -76,8 +95,6 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
         else okn = isvalid64(up, k);
         const unsigned badl = __ballot_sync(0xffffffffu, !okn);
         if (badl & (0xffffu << (16 * (kq & 1)))) face_mean(&s_uc[ml][0][0], V, up, k);
-#pragma unroll
-        for (int v = 0; v < V; ++v) uf[v] = a.u_in[((int64_t)v * E + qf) * NP + nf];
         // rotate into the face frame: component c of momentum (and field) -> original (d + c) % 3
         double rp[V], rf[V];
         rp[0] = up[0];
@@ -98,13 +115,18 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
                 rf[5 + c] = uf[5 + (d + c) % 3];
             }
         }
-        const double* uL = coarse_left ? rp : rf;
-        const double* uR = coarse_left ? rf : rp;
+        double uL[V], uR[V];   // by selection, not by pointer (which would put the arrays in local memory)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            uL[v] = coarse_left ? rp[v] : rf[v];
+            uR[v] = coarse_left ? rf[v] : rp[v];
+        }
         double F[V], Gf[V], Gc[V];
         double* out = a.mflux + ((5 * m + 1 + kq) * V) * NF + (i + NN * j);
         if (MHD) {
             const double ch = a.ctrl->glm_ch;
-            m_riemann_x<double>(a.surface_flux, uL, uR, F, k.kappa, k.mu0, ch);
+            if (a.surface_flux == NEMO_SURFFLUX_HLLD) m_hlld64(uL, uR, F, mhd64<true>(k, ch));
+            else m_rusanov64(uL, uR, F, mhd64<false>(k, ch));
             m_nc_x<double>(rf, uL, uR, Gf, k.mu0);
             m_nc_x<double>(rp, uL, uR, Gc, k.mu0);
 #pragma unroll
@@ -122,25 +144,29 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
         }
     }
     __syncthreads();
-    if (act && r < NF) {
-        const int aa = r & 3, bb = r >> 2;
-        double* out = a.mflux + (5 * m * V) * NF + r;
+    // projection, one axis at a time: thread (kq, jj, aa) the first, then the coarse nodes sum over the
+    // sub-faces and jj in the oracle's order
+    if (act) {
 #pragma unroll
         for (int v = 0; v < V; ++v) {
+            double in = 0.0;
+#pragma unroll
+            for (int ii = 0; ii < NN; ++ii) in = in + s_prj[s * NN * NN + i * NN + ii] * s_fs[ml][kq][v][ii + NN * j];
+            s_in[ml][v][r] = in;
+        }
+    }
+    __syncthreads();
+    if (act) {
+        double* out = a.mflux + (5 * m * V) * NF;
+        for (int p = r; p < NF * V; p += 64) {
+            const int v = p >> 4, aa = p & 3, bb = (p >> 2) & 3;
             double acc = 0.0;
 #pragma unroll
-            for (int t2 = 0; t2 < 2; ++t2)
+            for (int q = 0; q < 4; ++q)
 #pragma unroll
-                for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-                    for (int jj = 0; jj < NN; ++jj) {
-                        double in = 0.0;
-#pragma unroll
-                        for (int ii = 0; ii < NN; ++ii)
-                            in = in + k.prj[s2][aa * NN + ii] * s_fs[ml][s2 + 2 * t2][v][ii + NN * jj];
-                        acc = acc + k.prj[t2][bb * NN + jj] * in;
-                    }
-            out[v * NF] = acc;
+                for (int jj = 0; jj < NN; ++jj)
+                    acc = acc + s_prj[(q >> 1) * NN * NN + bb * NN + jj] * s_in[ml][v][q * NF + jj * NN + aa];
+            out[p] = acc;
         }
     }
     if (a.mflag) {  // publish: the mortar's five flux rows are complete for this epoch
