@@ -1,6 +1,7 @@
 // common.cuh -- layout, constants and small device helpers shared by the sm_100a kernels.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -24,11 +25,14 @@ struct Control {
     double dt_factor;                         // 0.5^(D-1) * cfl / (2*N_NODES - 1)
     int32_t ngroups;
     int32_t done;                             // all groups reached t_end
+    // the next five are read back together (RunStatus)
     int32_t error;                            // bit 0: bounded TMA wait expired; bit 1: non-finite dt;
                                               // bit 2: bounded wait on a mortar flag expired
     int32_t pad;
     unsigned long long nbad;                  // elements whose positivity repair failed
     unsigned long long steps;
+    unsigned long long nbad_mark;             // nbad and steps when the current call began
+    unsigned long long steps_mark;
     unsigned long long fallback;              // elements that used the modal fallback (learned indicator)
     double judge_sum;                         // sum |alpha_learned - alpha_modal| over judged elements
     unsigned long long judge_n;               // number of judged elements
@@ -42,6 +46,13 @@ struct Control {
     uint32_t exit_count;                      // persistent stage launches: CTAs finished
     uint32_t pad3;
 };
+
+// Control from `error` on, as the host reads it back after a run or a stage.
+struct RunStatus {
+    int32_t error, pad;
+    unsigned long long nbad, steps, nbad_mark, steps_mark;
+};
+static_assert(offsetof(Control, steps_mark) - offsetof(Control, error) == offsetof(RunStatus, steps_mark), "same layout");
 
 // Learned indicator: packed MLP weights (W1[32][12], b1[32], W2[32][32], b2[32], W3[32], b3)
 // followed by the lower and upper bounds of the 12 normalised inputs.

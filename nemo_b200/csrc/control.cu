@@ -19,7 +19,25 @@ __global__ void k_ctrl_reset(Control* c) {
 __global__ void k_ctrl_set_dt(Control* c, double dt) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < c->ngroups) c->dt[g] = dt;
-    if (g == 0) c->done = 0;
+    if (g == 0) {
+        c->done = 0;
+        c->nbad_mark = c->nbad;
+    }
+}
+
+// Start of a run: the extrema of the CFL bound reset, the end time set, not done, the step counter marked.
+__global__ void k_ctrl_begin(Control* c, double t_end) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < c->ngroups) {
+        c->dtmin_bits[g] = POS_INF_BITS;
+        c->lmax_bits[g] = 0ull;
+    }
+    if (g == 0) {
+        c->vmax_bits = 0ull;
+        c->t_end = t_end;
+        c->done = 0;
+        c->steps_mark = c->steps;
+    }
 }
 
 // hook_calc_timestep for the next step, from the CFL bounds accumulated by the previous
@@ -166,6 +184,11 @@ cudaError_t launch_unpack(double* u, double* alpha, const int32_t* idx, int64_t 
 
 cudaError_t launch_ctrl_reset(Control* c, cudaStream_t s) {
     k_ctrl_reset<<<MAX_GROUPS / 256, 256, 0, s>>>(c);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ctrl_begin(Control* c, double t_end, cudaStream_t s) {
+    k_ctrl_begin<<<MAX_GROUPS / 256, 256, 0, s>>>(c, t_end);
     return cudaGetLastError();
 }
 

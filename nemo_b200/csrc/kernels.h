@@ -138,6 +138,7 @@ cudaError_t launch_pack(const double* u, const double* alpha, const int32_t* idx
 cudaError_t launch_unpack(double* u, double* alpha, const int32_t* idx, int64_t n, int64_t E, int nv,
                           const double* buf, cudaStream_t s);
 cudaError_t launch_ctrl_reset(Control* c, cudaStream_t s);
+cudaError_t launch_ctrl_begin(Control* c, double t_end, cudaStream_t s);
 cudaError_t launch_ctrl_set_dt(Control* c, double dt, cudaStream_t s);
 cudaError_t launch_ctrl_step(Control* c, cudaStream_t s);
 cudaError_t launch_aos_to_soa(const double* aos, double* soa, int64_t E, int nv, cudaStream_t s);

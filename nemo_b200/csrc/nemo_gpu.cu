@@ -168,6 +168,18 @@ void build_host_ops(HostOps& h) {
 
 // ---- library state ----------------------------------------------------------------------------
 
+// What the host reads back from the control block after a call, in pinned memory: a copy into pageable
+// memory holds the host until it has run, once per value (us per call, 4^3 elements: stage 55 -> 33, one-step run 146 -> 99, time step 41 -> 35).
+struct HostStatus {
+    RunStatus run;
+    double t0;
+    unsigned long long dtmin_bits, lmax_bits, vmax_bits;
+    double totals[VMAX];
+    double glm[2];     // to the device: cleaning speed and damping of the coming step
+    int32_t done;
+    Control fresh;     // to the device: the control block of an uploaded state
+};
+
 struct Lib {
     bool inited = false;
     nemo_cfg cfg{};
@@ -180,7 +192,6 @@ struct Lib {
     int64_t E_own = 0;            // elements advanced by this process; [E_own, E) are ghost copies
     int64_t n_interior = 0;       // owned elements [0, n_interior) read no ghost data (0: no split)
     bool split_open = false;      // a stage's interior part is enqueued, its boundary part not yet
-    unsigned long long nbad_mark = 0;  // repair-failure count before the open split stage (host copy)
     int V = 5;
     bool has_mesh = false, has_state = false;
     int ngroups = 1;
@@ -206,6 +217,7 @@ struct Lib {
     Control* ctrl = nullptr;
     double* part = nullptr;       // totals partials [V][E]
     double* tot = nullptr;        // totals [10]
+    HostStatus* host = nullptr;   // pinned
     int cur = 0;                  // u[cur] holds the state, alpha[cur] its raw indicator
     bool prepared = false;        // alpha[cur] and the CFL bound in ctrl are valid for u[cur]
     bool reg_valid = false;
@@ -471,10 +483,11 @@ int prepare_if_needed() {
     return NEMO_OK;
 }
 
+// Waits for the stream; g.host->run is then the control block's state after everything enqueued.
 int check_ctrl_error() {
-    int32_t err = 0;
-    CK(cudaMemcpyAsync(&err, &g.ctrl->error, sizeof err, cudaMemcpyDeviceToHost, g.stream));
+    CK(cudaMemcpyAsync(&g.host->run, &g.ctrl->error, sizeof(RunStatus), cudaMemcpyDeviceToHost, g.stream));
     CK(cudaStreamSynchronize(g.stream));
+    const int32_t err = g.host->run.error;
     if (err & 1) return fail(NEMO_ERR_CUDA, "a bounded device wait expired (TMA copy did not complete)");
     if (err & 2) return fail(NEMO_ERR_NONFINITE, "non-finite or negative time step");
     if (err & 4) return fail(NEMO_ERR_CUDA, "a bounded wait on a mortar flag expired");
@@ -714,6 +727,7 @@ int nemo_gpu_init(const nemo_cfg* cfg) {
     CK(cudaMalloc(&g.ctrl, sizeof(Control)));
     CK(cudaMemset(g.ctrl, 0, sizeof(Control)));
     CK(cudaMalloc(&g.tot, 16 * sizeof(double)));
+    if (!g.host) CK(cudaHostAlloc((void**)&g.host, sizeof(HostStatus), cudaHostAllocDefault));
     CK(cudaMalloc(&g.mlp32, sizeof(float) * (MLP_NPACK + 8 + MLP_NT)));
     CK(cudaMalloc(&g.mlp64, sizeof(double) * MLP_NPACK));
     g.mlp_ready = false;
@@ -979,8 +993,8 @@ int nemo_gpu_upload_state(const double* host, int64_t stride) {
     CK(launch_aos_to_soa(g.stagebuf, g.u[0], g.E, g.V, g.stream));
     CK(cudaMemsetAsync(g.reg, 0, row * g.E, g.stream));
     // reset the simulation time and counters
-    const Control c = fresh_control();
-    CK(cudaMemcpyAsync(g.ctrl, &c, sizeof c, cudaMemcpyHostToDevice, g.stream));
+    g.host->fresh = fresh_control();
+    CK(cudaMemcpyAsync(g.ctrl, &g.host->fresh, sizeof(Control), cudaMemcpyHostToDevice, g.stream));
     CK(cudaStreamSynchronize(g.stream));
     g.has_state = true;
     g.prepared = false;
@@ -1163,24 +1177,21 @@ int nemo_gpu_calc_timestep(double cfl, double* dt_out, double* lmax_out) {
     if (!(cfl > 0.0)) return fail(NEMO_ERR_ARG, "cfl must be positive");
     CK(launch_ctrl_reset(g.ctrl, g.stream));
     CK(launch_prepare(true, g.stream));
-    unsigned long long bits[2];
-    CK(cudaMemcpyAsync(&bits[0], &g.ctrl->dtmin_bits[0], 8, cudaMemcpyDeviceToHost, g.stream));
-    CK(cudaMemcpyAsync(&bits[1], &g.ctrl->lmax_bits[0], 8, cudaMemcpyDeviceToHost, g.stream));
+    CK(cudaMemcpyAsync(&g.host->dtmin_bits, &g.ctrl->dtmin_bits[0], 8, cudaMemcpyDeviceToHost, g.stream));
+    CK(cudaMemcpyAsync(&g.host->lmax_bits, &g.ctrl->lmax_bits[0], 8, cudaMemcpyDeviceToHost, g.stream));
+    if (is_mhd()) CK(cudaMemcpyAsync(&g.host->vmax_bits, &g.ctrl->vmax_bits, 8, cudaMemcpyDeviceToHost, g.stream));
     CK(cudaStreamSynchronize(g.stream));
     double dtmin, lmax;
-    std::memcpy(&dtmin, &bits[0], 8);
-    std::memcpy(&lmax, &bits[1], 8);
+    std::memcpy(&dtmin, &g.host->dtmin_bits, 8);
+    std::memcpy(&lmax, &g.host->lmax_bits, 8);
     const double dt = 0.25 * cfl / (double)(2 * NN - 1) * dtmin;
     if (!std::isfinite(dt) || !(dt > 0.0)) return fail(NEMO_ERR_NONFINITE, "time step %g is not positive and finite", dt);
     if (is_mhd()) {  // GLM cleaning speed and damping for the coming step (kernel_timestep_mod.f90:338-344)
-        unsigned long long vb = 0;
-        CK(cudaMemcpy(&vb, &g.ctrl->vmax_bits, 8, cudaMemcpyDeviceToHost));
         double vmax;
-        std::memcpy(&vmax, &vb, 8);
-        const double gch = 2.0 * std::fabs(lmax - vmax);
-        const double gal = gch / 0.18;
-        CK(cudaMemcpy(&g.ctrl->glm_ch, &gch, 8, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(&g.ctrl->glm_alpha, &gal, 8, cudaMemcpyHostToDevice));
+        std::memcpy(&vmax, &g.host->vmax_bits, 8);
+        g.host->glm[0] = 2.0 * std::fabs(lmax - vmax);
+        g.host->glm[1] = g.host->glm[0] / 0.18;
+        CK(cudaMemcpyAsync(&g.ctrl->glm_ch, g.host->glm, 16, cudaMemcpyHostToDevice, g.stream));
     }
     if (dt_out) *dt_out = dt;
     if (lmax_out) *lmax_out = lmax;
@@ -1194,15 +1205,13 @@ int nemo_gpu_stage(int32_t stage, double dt, double t_stage, int32_t* nbad_out) 
     (void)t_stage;
     if (stage < 1 || stage > 5) return fail(NEMO_ERR_ARG, "stage must be 1..5");
     if (!(dt >= 0.0) || !std::isfinite(dt)) return fail(NEMO_ERR_ARG, "dt must be finite and >= 0");
-    unsigned long long nb0 = 0, nb1 = 0;
-    CK(cudaMemcpyAsync(&nb0, &g.ctrl->nbad, 8, cudaMemcpyDeviceToHost, g.stream));
     if ((st = prepare_if_needed())) return st;
-    CK(launch_ctrl_set_dt(g.ctrl, dt, g.stream));
+    CK(launch_ctrl_set_dt(g.ctrl, dt, g.stream));   // marks the repair-failure count
     CK(launch_stage(stage - 1, g.stream));
-    CK(cudaMemcpyAsync(&nb1, &g.ctrl->nbad, 8, cudaMemcpyDeviceToHost, g.stream));
     if ((st = check_ctrl_error())) return st;
-    if (nbad_out) *nbad_out = (int32_t)(nb1 - nb0);
-    if (nb1 > nb0) return fail(NEMO_ERR_REPAIR, "positivity repair failed on %llu elements", nb1 - nb0);
+    const unsigned long long failed = g.host->run.nbad - g.host->run.nbad_mark;
+    if (nbad_out) *nbad_out = (int32_t)failed;
+    if (failed > 0) return fail(NEMO_ERR_REPAIR, "positivity repair failed on %llu elements", failed);
     return NEMO_OK;
 }
 
@@ -1231,8 +1240,7 @@ int nemo_gpu_stage_interior(int32_t stage, double dt) {
     if (!(dt >= 0.0) || !std::isfinite(dt)) return fail(NEMO_ERR_ARG, "dt must be finite and >= 0");
     if (g.tune_mode == 1) return fail(NEMO_ERR_STATE, "split stages need the grid schedule (nemo_gpu_set_schedule 0)");
     if ((st = prepare_if_needed())) return st;
-    CK(cudaMemcpyAsync(&g.nbad_mark, &g.ctrl->nbad, 8, cudaMemcpyDeviceToHost, g.stream));
-    CK(launch_ctrl_set_dt(g.ctrl, dt, g.stream));
+    CK(launch_ctrl_set_dt(g.ctrl, dt, g.stream));   // marks the repair-failure count
     // the interior part advances the clock only when there is no boundary part
     CK(launch_stage_part(stage - 1, 0, g.n_interior, g.n_interior == g.E_own, g.stream));
     g.split_open = true;
@@ -1247,11 +1255,10 @@ int nemo_gpu_stage_boundary(int32_t stage, double dt, int32_t* nbad_out) {
     g.split_open = false;
     if (g.E_own > g.n_interior) CK(launch_stage_part(stage - 1, g.n_interior, g.E_own, true, g.stream));
     g.cur ^= 1;
-    unsigned long long nb1 = 0;
-    CK(cudaMemcpyAsync(&nb1, &g.ctrl->nbad, 8, cudaMemcpyDeviceToHost, g.stream));
     if ((st = check_ctrl_error())) return st;
-    if (nbad_out) *nbad_out = (int32_t)(nb1 - g.nbad_mark);
-    if (nb1 > g.nbad_mark) return fail(NEMO_ERR_REPAIR, "positivity repair failed on %llu elements", nb1 - g.nbad_mark);
+    const unsigned long long failed = g.host->run.nbad - g.host->run.nbad_mark;
+    if (nbad_out) *nbad_out = (int32_t)failed;
+    if (failed > 0) return fail(NEMO_ERR_REPAIR, "positivity repair failed on %llu elements", failed);
     return NEMO_OK;
 }
 
@@ -1313,15 +1320,11 @@ int nemo_gpu_run(int64_t nsteps, double t_end, double* t_out, int64_t* steps_out
     int st = ensure_ready();
     if (st) return st;
     if (nsteps <= 0 && !(t_end > 0.0)) return fail(NEMO_ERR_ARG, "give nsteps > 0 or t_end > 0");
-    g.prepared = false;  // the CFL bound must belong to the current state
-    if ((st = prepare_if_needed())) return st;
+    // the CFL bound must belong to the current state
+    CK(launch_ctrl_begin(g.ctrl, t_end, g.stream));
+    CK(launch_prepare(true, g.stream));
+    g.prepared = true;
     const int64_t prep_launches = 2;
-    CK(cudaMemcpyAsync(&g.ctrl->t_end, &t_end, sizeof(double), cudaMemcpyHostToDevice, g.stream));
-    const int32_t zero = 0;
-    CK(cudaMemcpyAsync(&g.ctrl->done, &zero, sizeof zero, cudaMemcpyHostToDevice, g.stream));
-    unsigned long long steps0 = 0, steps1 = 0;
-    CK(cudaMemcpyAsync(&steps0, &g.ctrl->steps, 8, cudaMemcpyDeviceToHost, g.stream));
-    CK(cudaStreamSynchronize(g.stream));
     const int start_cur = g.cur;
     int64_t issued = 0;
     const int64_t limit = nsteps > 0 ? nsteps : INT64_MAX;
@@ -1372,19 +1375,16 @@ int nemo_gpu_run(int64_t nsteps, double t_end, double* t_out, int64_t* steps_out
         }
         issued += chunk;
         if (t_end > 0.0) {
-            int32_t done = 0;
-            CK(cudaMemcpyAsync(&done, &g.ctrl->done, sizeof done, cudaMemcpyDeviceToHost, g.stream));
+            CK(cudaMemcpyAsync(&g.host->done, &g.ctrl->done, sizeof g.host->done, cudaMemcpyDeviceToHost, g.stream));
             CK(cudaStreamSynchronize(g.stream));
-            if (done) break;
+            if (g.host->done) break;
         }
     }
-    CK(cudaMemcpyAsync(&steps1, &g.ctrl->steps, 8, cudaMemcpyDeviceToHost, g.stream));
-    double t0 = 0.0;
-    CK(cudaMemcpyAsync(&t0, &g.ctrl->t[0], 8, cudaMemcpyDeviceToHost, g.stream));
+    CK(cudaMemcpyAsync(&g.host->t0, &g.ctrl->t[0], 8, cudaMemcpyDeviceToHost, g.stream));
     if ((st = check_ctrl_error())) return st;
-    const int64_t done_steps = (int64_t)(steps1 - steps0);
+    const int64_t done_steps = (int64_t)(g.host->run.steps - g.host->run.steps_mark);
     g.cur = start_cur ^ (int)(done_steps & 1);
-    if (t_out) *t_out = t0;
+    if (t_out) *t_out = g.host->t0;
     if (steps_out) *steps_out = done_steps;
     return NEMO_OK;
 }
@@ -1428,10 +1428,9 @@ int nemo_gpu_totals(double* out) {
     if (st) return st;
     if (!out) return fail(NEMO_ERR_ARG, "out is NULL");
     CK(launch_totals64(g.u[g.cur], g.delta, g.E, g.E_own, g.V, g.part, g.tot, g.stream));
-    double tmp[16] = {0};
-    CK(cudaMemcpyAsync(tmp, g.tot, sizeof(double) * g.V, cudaMemcpyDeviceToHost, g.stream));
+    CK(cudaMemcpyAsync(g.host->totals, g.tot, sizeof(double) * g.V, cudaMemcpyDeviceToHost, g.stream));
     CK(cudaStreamSynchronize(g.stream));
-    for (int v = 0; v < 10; ++v) out[v] = v < g.V ? tmp[v] : 0.0;
+    for (int v = 0; v < 10; ++v) out[v] = v < g.V ? g.host->totals[v] : 0.0;
     return NEMO_OK;
 }
 
@@ -1816,6 +1815,8 @@ int nemo_gpu_finalize(void) {
     if (g.out_stream) cudaStreamDestroy(g.out_stream);
     g.out_stream = nullptr;
     g.out_next = 0;
+    if (g.host) cudaFreeHost(g.host);
+    g.host = nullptr;
     g.ctrl = nullptr;
     g.tot = nullptr;
     g.mlp32 = nullptr;
