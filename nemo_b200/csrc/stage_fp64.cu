@@ -75,6 +75,13 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 
 __device__ __forceinline__ double silu64(double x) { return x / (1.0 + pexp64(-x)); }
 
+// Barrier of one element's 64 threads: of the CTA, or (ND = 3, see k_stage_euler64) of group g of it
+template <int ND>
+__device__ __forceinline__ void group_sync(int g) {
+    if (ND == 1) __syncthreads();
+    else asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory");
+}
+
 // maximum over the warp by bit patterns (non-negative values; a NaN counts as the largest)
 __device__ __forceinline__ unsigned long long wmax64(double x) {
     unsigned long long v = (unsigned long long)__double_as_longlong(x);
@@ -116,6 +123,7 @@ __device__ __forceinline__ void load_rot64(const double* u, const double* m0, co
 
 // Modal coefficients of the nodal values q (one per thread) into cm[64]: x and y inside a warp, z
 // across the element's two warps; t1, t2 are [64] scratch.
+template <int ND>
 __device__ __forceinline__ double modal64(double q, double* t1, double* t2, const double* vi, int n) {
     const int x = n & 3, y = (n >> 2) & 3, z = n >> 4;
     t1[n] = q;
@@ -130,7 +138,7 @@ __device__ __forceinline__ double modal64(double q, double* t1, double* t2, cons
     for (int j = 0; j < NN; ++j) s = s + vi[y * NN + j] * t2[nidx(x, j, z)];
     __syncwarp();
     t1[n] = s;
-    __syncthreads();
+    group_sync<ND>(0);
     s = 0.0;
 #pragma unroll
     for (int k = 0; k < NN; ++k) s = s + vi[z * NN + k] * t1[nidx(x, y, k)];
@@ -142,7 +150,7 @@ __device__ __forceinline__ double modal64(double q, double* t1, double* t2, cons
 // learned indicator with the modal one as fallback and judge) and, if requested, the per-element CFL bound
 // from the wave speeds lambda(d).  sp: scratch of the element, six [64] arrays.  Sums run in the oracle's
 // serial order.
-template <typename Lambda>
+template <int ND, typename Lambda>
 __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, double pr, double* sp, const double* vi,
                                            unsigned long long (*s_lam)[4], int64_t e, int n, const OpConsts& k,
                                            Lambda lambda) {
@@ -150,12 +158,12 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
     const int lane = n & 31, w = n >> 5;
     if (a.alpha_out) {
         double* e2 = sp + 2 * NP;   // [3][64]: squared modes, those of order < N, those of order < N-1
-        const double m = modal64(rho * pr, sp, sp + NP, vi, n);
+        const double m = modal64<ND>(rho * pr, sp, sp + NP, vi, n);
         const int top = max(max(n & 3, (n >> 2) & 3), n >> 4);
         e2[n] = m * m;
         e2[NP + n] = top < NN - 1 ? m * m : 0.0;
         e2[2 * NP + n] = top < NN - 2 ? m * m : 0.0;
-        __syncthreads();
+        group_sync<ND>(0);
         double am = 0.0;
         if (w == 0) {
             // one sum per lane 0..2, in mode order (the zeros change nothing)
@@ -179,16 +187,16 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
             double* er = sp + 3 * NP;
             double* ep = sp + 4 * NP;
             double* np = sp + 5 * NP;
-            __syncthreads();   // the sums above are done with e2
-            const double mr = modal64(rho, sp, sp + NP, vi, n);
-            __syncthreads();
-            const double mp = modal64(pr, sp, sp + NP, vi, n);
+            group_sync<ND>(0);   // the sums above are done with e2
+            const double mr = modal64<ND>(rho, sp, sp + NP, vi, n);
+            group_sync<ND>(0);
+            const double mp = modal64<ND>(pr, sp, sp + NP, vi, n);
             er[n] = mr * mr;
             ep[n] = mp * mp;
             np[n] = pr;
-            __syncthreads();
+            group_sync<ND>(0);
             sp[n] = rho;     // nodal rho (the transform scratch is dead)
-            __syncthreads();
+            group_sync<ND>(0);
             if (w == 0) {
                 double* feat = sp + NP;      // [12]
                 double* h1 = sp + NP + 16;   // [32]
@@ -255,7 +263,7 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
             const unsigned long long lam = wmax64(lambda(dd));
             if (lane == 0) s_lam[w][dd] = lam;
         }
-        __syncthreads();
+        group_sync<ND>(0);
         if (n == 0) {
             const double lf = __longlong_as_double((long long)max(s_lam[0][0], s_lam[1][0]));
             const double lg = __longlong_as_double((long long)max(s_lam[0][1], s_lam[1][1]));
@@ -270,8 +278,11 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
 
 }  // namespace
 
-template <bool BLEND, bool RHS_ONLY, bool FAST>
-__global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
+// ND directions at a time, each by a group of 64 threads with its own flux arrays.  ND = 1 (64 threads) packs
+// an SM with elements; ND = 3 (192 threads) runs an element's directions side by side, which shortens the
+// element (26 k cycles alone, 18 k of them the directions) when there are too few to fill the SMs anyway.
+template <int ND, bool BLEND, bool RHS_ONLY, bool FAST>
+__global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageArgs a) {
     extern __shared__ __align__(16) double smem[];
     __shared__ double s_S[NN * NN], s_winv[NN], s_vi[NN * NN];   // operator rows, indexed per thread
     __shared__ double s_alpha;
@@ -281,44 +292,50 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
 
     const OpConsts& k = c_ops64;
     Control* ctrl = a.ctrl;
-    const int n = threadIdx.x, lane = n & 31, w = n >> 5;
+    const int tid = threadIdx.x, dg = ND == 1 ? 0 : tid / TPE, n = ND == 1 ? tid : tid % TPE, lane = n & 31, w = n >> 5;
     const int64_t E = a.E;
     const int64_t e = a.E_begin + blockIdx.x;
-    if (n < NN * NN) {
-        s_S[n] = k.S[n];
-        s_vi[n] = k.Vinv[n];
-        if (n < NN) s_winv[n] = k.winv[n];
+    if (tid < NN * NN) {
+        s_S[tid] = k.S[tid];
+        s_vi[tid] = k.Vinv[tid];
+        if (tid < NN) s_winv[tid] = k.winv[tid];
     }
-    // faces p of the neighbour traces this thread fetches, p = n and (warp 0) n + 64
-    const int32_t nes[2] = {__ldg(a.nbr + e * 6 + (n >> 4)), n < 6 * NF - TPE ? __ldg(a.nbr + e * 6 + 4 + (n >> 4)) : -1};
+    // trace nodes p of the six faces this thread fetches: p = tid and, with 64 threads, (warp 0) tid + 64
+    constexpr int FETCH = ND == 1 ? 2 : 1;
+    int32_t nes[FETCH];
+#pragma unroll
+    for (int r = 0; r < FETCH; ++r)
+        nes[r] = (ND == 1 && r == 0) || tid + r * TPE < 6 * NF ? __ldg(a.nbr + e * 6 + 4 * r + (tid >> 4)) : -1;
     dep_sync();
     if (!RHS_ONLY && ctrl->done) return;
     double* const su = smem + O_SU;
     double* const sp = smem + O_SP;
     double* const tr = smem + O_TR;
-    double* const sF = smem + O_SF;
-    double* const sV = smem + O_SV;
+    constexpr int PER = (BLEND ? ELEM_BLEND : ELEM_PLAIN) - O_SF;   // flux arrays of a direction
+    double* const sF = smem + O_SF + dg * PER;
+    double* const sV = sF + (O_SV - O_SF);
+    double* const sR = smem + O_SF + ND * PER;                       // ND = 3: [2][V][64] rhs terms of y and z
 
     double q[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
     auto epilogue = [&]() {
-        epilogue64(a, q[0], pressure64(q, k), sp, s_vi, s_lam, e, n, k, [&](int dd) {
+        epilogue64<ND>(a, q[0], pressure64(q, k), sp, s_vi, s_lam, e, n, k, [&](int dd) {
             const double rr[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
             return xlambda64(rr, k);
         });
     };
     if (a.prep_only) {
         __syncthreads();
-        epilogue();
+        if (dg == 0) epilogue();
         return;
     }
 
     // neighbour traces (or mortar flux rows) of the 96 face nodes, asynchronously
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int p = n + r * TPE, f = p >> 4, ab = p & 15;
-        if (p >= 6 * NF) break;
+    for (int r = 0; r < FETCH; ++r) {
+        const int p = tid + r * TPE, f = p >> 4, ab = p & 15;
+        if (!(ND == 1 && r == 0) && p >= 6 * NF) break;
         const int32_t ne = nes[r];
         if (ab == 0) s_nbr[f] = ne;
         if (ne >= 0) {
@@ -331,23 +348,26 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
             for (int v = 0; v < V; ++v) cp_async8(tr + v * 6 * NF + p, g + v * NF);
         }
     }
-    if (!RHS_ONLY && a.stage > 0 && n < 4 * V)   // the register rows (four lines each), needed at the end
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.reg + ((int64_t)(n >> 2) * E + e) * NP + 16 * (n & 3)));
-    if (n == 0) s_bad = 0;
-    if (BLEND && w == 0) smooth_alpha64(a, e, lane, &s_alpha);
+    if (!RHS_ONLY && a.stage > 0 && tid < 4 * V)   // the register rows (four lines each), needed at the end
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.reg + ((int64_t)(tid >> 2) * E + e) * NP + 16 * (tid & 3)));
+    if (tid == 0) s_bad = 0;
+    if (BLEND && tid < 32) smooth_alpha64(a, e, lane, &s_alpha);
 
     // per-node primitives: velocities and, per direction d, beta_d = rho/(2 p_d) where p_d is the
     // pressure of the state rotated into direction d (the reference evaluates the two-point flux on
     // the rotated state, so the kinetic-energy sum runs in the rotated component order)
     const int pn = phys(n);
-#pragma unroll
-    for (int v = 0; v < V; ++v) su[v * NP + pn] = q[v];
     const Rcp64 ir = rcp64r(q[0]);
-    sp[6 * NP + pn] = ir.y;
+    if (dg == 0) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) sp[c * NP + pn] = quot64(q[1 + c], ir);
+        for (int v = 0; v < V; ++v) su[v * NP + pn] = q[v];
+        sp[6 * NP + pn] = ir.y;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sp[c * NP + pn] = quot64(q[1 + c], ir);
+    }
 #pragma unroll
     for (int dd = 0; dd < 3; ++dd) {
+        if (ND == 3 && dd != dg) continue;
         const double r[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
         sp[(3 + dd) * NP + pn] = div64(0.5 * q[0], pressure64(r, ir, k));
     }
@@ -361,7 +381,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
 #pragma unroll
     for (int v = 0; v < V; ++v) R[v] = 0.0;
 #pragma unroll 1
-    for (int d = 0; d < 3; ++d) {
+    for (int d = dg; d < (ND == 1 ? 3 : dg + 1); ++d) {
         const int c0 = d, c1 = d == 2 ? 0 : d + 1, c2 = d == 0 ? 2 : d - 1;
         const double *m0 = su + (1 + c0) * NP, *m1 = su + (1 + c1) * NP, *m2 = su + (1 + c2) * NP;   // momenta
         constexpr int VEL = O_SP - NP, BETA = O_SP + 2 * NP;   // from a momentum to its velocity, to its beta
@@ -423,7 +443,7 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
                 for (int v = 0; v < V; ++v) sV[(v * (NN - 1) + 2 * (rt - 1) + hi) * FROW + ab] = F[v];
             }
         }
-        __syncthreads();
+        group_sync<ND>(dg);
         // ---- the node's terms: its three pairs in ascending order of the other node, lift, FV, blend
         const int pos = (n >> (2 * d)) & 3;
         const int ab = d == 0 ? n >> 2 : (d == 1 ? (n & 3) | ((n >> 4) << 2) : n & 15);
@@ -459,15 +479,34 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
             }
         }
         const double cd = __ldg(a.cdel + e * 3 + d);
-        double r[V];
+        if (ND == 3) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) r[v] = d == 0 ? cd * t[v] : R[v] + cd * t[v];
-        R[0] = r[0];
-        R[1] = r[2];
-        R[2] = r[3];
-        R[3] = r[1];
-        R[4] = r[4];
+            for (int v = 0; v < V; ++v) R[v] = cd * t[v];
+            if (d > 0) {   // x keeps its terms in registers
+                double* o = sR + (d - 1) * V * NP + n;
+                o[0] = R[0];
+                o[(1 + c0) * NP] = R[1];
+                o[(1 + c1) * NP] = R[2];
+                o[(1 + c2) * NP] = R[3];
+                o[4 * NP] = R[4];
+            }
+        } else {
+            double r[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) r[v] = d == 0 ? cd * t[v] : R[v] + cd * t[v];
+            R[0] = r[0];
+            R[1] = r[2];
+            R[2] = r[3];
+            R[3] = r[1];
+            R[4] = r[4];
+            __syncthreads();
+        }
+    }
+    if (ND == 3) {
         __syncthreads();
+        if (dg != 0) return;   // the rest is group 0's
+#pragma unroll
+        for (int v = 0; v < V; ++v) R[v] = (R[v] + sR[v * NP + n]) + sR[(V + v) * NP + n];
     }
 
     // ---- rhs, LSRK register and state update
@@ -492,18 +531,18 @@ __global__ void __launch_bounds__(TPE, CTAS64) k_stage_euler64(StageArgs a) {
     }
     if (a.positivity) {
         if (!isvalid64(q, k)) s_bad = 1;
-        __syncthreads();
+        group_sync<ND>(0);
         if (s_bad) {
             // lanes 0..15 of warp 0 repair the element together on a copy in node order (same
             // arithmetic and order as the serial dgfv_repair_3d)
 #pragma unroll
             for (int v = 0; v < V; ++v) sF[v * NP + n] = q[v];
-            __syncthreads();
+            group_sync<ND>(0);
             if (n < 16) {
                 const bool repaired = repair_elem16<1>(sF, 0, n, k);
                 if (!repaired && n == 0) atomicAdd(&ctrl->nbad, 1ull);
             }
-            __syncthreads();
+            group_sync<ND>(0);
 #pragma unroll
             for (int v = 0; v < V; ++v) q[v] = sF[v * NP + n];
         }
@@ -593,24 +632,38 @@ __global__ void __launch_bounds__(TSUM) k_totals_sum64(const double* __restrict_
 // ---------------------------------------------------------------------------------------------
 // launchers
 
-static int smem64(bool blend) { return (blend ? ELEM_BLEND : ELEM_PLAIN) * (int)sizeof(double); }
+static int smem64(int nd, bool blend) {
+    return (O_SF + nd * ((blend ? ELEM_BLEND : ELEM_PLAIN) - O_SF) + (nd == 3 ? 2 * V * NP : 0)) * (int)sizeof(double);
+}
 
-cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s) {
-    if (a.E_own <= a.E_begin) return cudaSuccess;
-    const unsigned grid = (unsigned)(a.E_own - a.E_begin);
-    const int smem = smem64(blend);
+// Up to so many elements, what the SMs hold at once with ND = 1, three directions at a time (set by the setup).
+// B200, us per stage, blended: 64 elements 14.3 -> 9.2, 216 15.0 -> 10.6, 512 17 -> 14, 910 22.6 -> 21.6, 1584
+// 31.0 -> 30.5; beyond, the wider CTAs' idle warps cost more than they save: 2197 39.1 -> 39.2, 4096 59.6 -> 65.8,
+// 32768 380 -> 491.
+static int64_t wide_elems64 = 0;
+
+template <int ND>
+static cudaError_t launch64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s) {
+    const unsigned grid = (unsigned)(a.E_own - a.E_begin), nt = ND * TPE;
+    const int smem = smem64(ND, blend);
     // the specialised kernel for HLLC faces and Chandrashekar pairs, the general one for the rest
     const bool fast = a.surface_flux == NEMO_SURFFLUX_HLLC && a.volume_flux == NEMO_VOLFLUX_CHANDRASHEKAR;
     if (rhs_only) {
-        if (blend) return launch_dep(k_stage_euler64<true, true, false>, grid, TPE, smem, s, a);
-        return launch_dep(k_stage_euler64<false, true, false>, grid, TPE, smem, s, a);
+        if (blend) return launch_dep(k_stage_euler64<ND, true, true, false>, grid, nt, smem, s, a);
+        return launch_dep(k_stage_euler64<ND, false, true, false>, grid, nt, smem, s, a);
     }
     if (fast) {
-        if (blend) return launch_dep(k_stage_euler64<true, false, true>, grid, TPE, smem, s, a);
-        return launch_dep(k_stage_euler64<false, false, true>, grid, TPE, smem, s, a);
+        if (blend) return launch_dep(k_stage_euler64<ND, true, false, true>, grid, nt, smem, s, a);
+        return launch_dep(k_stage_euler64<ND, false, false, true>, grid, nt, smem, s, a);
     }
-    if (blend) return launch_dep(k_stage_euler64<true, false, false>, grid, TPE, smem, s, a);
-    return launch_dep(k_stage_euler64<false, false, false>, grid, TPE, smem, s, a);
+    if (blend) return launch_dep(k_stage_euler64<ND, true, false, false>, grid, nt, smem, s, a);
+    return launch_dep(k_stage_euler64<ND, false, false, false>, grid, nt, smem, s, a);
+}
+
+cudaError_t launch_stage_euler64(const StageArgs& a, bool blend, bool rhs_only, cudaStream_t s) {
+    const int64_t n = a.E_own - a.E_begin;
+    if (n <= 0) return cudaSuccess;
+    return n <= wide_elems64 ? launch64<3>(a, blend, rhs_only, s) : launch64<1>(a, blend, rhs_only, s);
 }
 
 // The largest carveout: twelve elements take 220 KB of an SM's shared memory, and the kernel reads
@@ -622,14 +675,26 @@ static cudaError_t attrs64(K kernel, int smem) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
 }
 
+template <int ND>
+static cudaError_t setup64() {
+    cudaError_t err;
+    const int sb = smem64(ND, true), sn = smem64(ND, false);
+    if ((err = attrs64(k_stage_euler64<ND, true, true, false>, sb)) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<ND, false, true, false>, sn)) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<ND, true, false, false>, sb)) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<ND, false, false, false>, sn)) != cudaSuccess) return err;
+    if ((err = attrs64(k_stage_euler64<ND, true, false, true>, sb)) != cudaSuccess) return err;
+    return attrs64(k_stage_euler64<ND, false, false, true>, sn);
+}
+
 cudaError_t setup_stage_euler64(const OpConsts& ops) {
     cudaError_t err;
-    if ((err = attrs64(k_stage_euler64<true, true, false>, smem64(true))) != cudaSuccess) return err;
-    if ((err = attrs64(k_stage_euler64<false, true, false>, smem64(false))) != cudaSuccess) return err;
-    if ((err = attrs64(k_stage_euler64<true, false, false>, smem64(true))) != cudaSuccess) return err;
-    if ((err = attrs64(k_stage_euler64<false, false, false>, smem64(false))) != cudaSuccess) return err;
-    if ((err = attrs64(k_stage_euler64<true, false, true>, smem64(true))) != cudaSuccess) return err;
-    if ((err = attrs64(k_stage_euler64<false, false, true>, smem64(false))) != cudaSuccess) return err;
+    int dev = 0, nsm = 0;
+    if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
+    if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
+    wide_elems64 = CTAS64 * (int64_t)nsm;
+    if ((err = setup64<1>()) != cudaSuccess) return err;
+    if ((err = setup64<3>()) != cudaSuccess) return err;
     return cudaMemcpyToSymbol(c_ops64, &ops, sizeof(OpConsts));
 }
 

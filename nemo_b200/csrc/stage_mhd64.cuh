@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(TPE, mhd64k::CTAS) k_stage_mhd64(StageArgs a) 
 #pragma unroll
     for (int v = 0; v < MV; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
     auto epilogue = [&]() {
-        epilogue64(a, q[0], m_pressure<double>(q, k.kappa, FAST ? 1.0 : k.mu0), sp, s_vi, s_lam, e, n, k,
+        epilogue64<1>(a, q[0], m_pressure<double>(q, k.kappa, FAST ? 1.0 : k.mu0), sp, s_vi, s_lam, e, n, k,
                    [&](int dd) {
                        const double rr[MV] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4],
                                               q[5 + dd], q[5 + (dd + 1) % 3], q[5 + (dd + 2) % 3], q[8]};

@@ -124,3 +124,31 @@ def test_totals_at_chunk_edges(box):
         s.upload(u)
         assert np.array_equal(s.totals(), orc.Oracle.for_mesh(c, m).totals(u)[: u.shape[0]])
         s.finalize()
+
+
+@pytest.mark.parametrize("over", [0, 1])
+@pytest.mark.parametrize("form", ["special", "general", "learned"])
+def test_either_side_of_the_wide_kernels_limit(over, form):
+    """The largest mesh that takes three directions at a time (12 elements per SM) and one element more, with every
+    kind of kernel: specialised, general, learned indicator, and the rhs kernel."""
+    import torch
+    from nemo_b200 import learned
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m = mesh.brick(12 * sms + over, 1, 1)
+    u = setups.smooth_random(m, seed=3)
+    u[:, :, 17] *= 1.5
+    kw = dict(indicator=abi.IND_LEARNED if form == "learned" else abi.IND_MODAL, positivity=1)
+    if form == "general":
+        kw.update(surface_flux=abi.SURFFLUX_RUSANOV, volume_flux=abi.VOLFLUX_CENTRAL)
+    c = abi.default_cfg(**kw)
+    s = Solver(c, m)
+    if form == "learned":
+        learned.install()
+        w, lo, hi, _ = learned.load()
+        orc.set_mlp(learned.bf16_round(w), lo, hi)
+    o = orc.Oracle.for_mesh(c, m)
+    s.upload(u)
+    assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)))
+    t, _ = s.run(nsteps=2)
+    ref, tr, _, _ = o.run(u, nsteps=2)
+    assert t == tr and np.array_equal(s.download(), ref)
