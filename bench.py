@@ -392,7 +392,7 @@ def measure_secondary(wl, args, peaks, torch, ctypes, abi):
         out[key] = {"value": dof_per_step * args.steps / (ms * 1e-3), "unit": "DOF-updates/s",
                     "ms_per_step": ms / args.steps, "avg_stage_ms": avg_s * 1e3, "schedule": sched,
                     "kernel": ("k_stage_mhd<float>" if mhd else "k_stage_euler32") if prec else
-                              ("k_stage_mhd<double>" if mhd else "k_stage_euler64"),
+                              ("k_stage_mhd64" if mhd else "k_stage_euler64"),
                     "roofline": rf}
     out["chosen_form_speedup"] = out["fp32_modal"]["value"] / out["fp64_modal"]["value"]
     return out
@@ -744,7 +744,7 @@ def main():  # noqa: C901
             forms[key] = {"value": r["value"], "unit": "DOF-updates/s", "ms_per_step": r["ms"] / args.steps,
                           "avg_stage_ms": r["avg_stage_ms"], "schedule": r["schedule"],
                           "roofline": r["roofline"], "chosen_form_speedup": value / r["value"]}
-        forms["fp64_modal"]["kernel"] = "k_stage_mhd<double>" if mhd else "k_stage_euler64"
+        forms["fp64_modal"]["kernel"] = "k_stage_mhd64" if mhd else "k_stage_euler64"
         line["plain_fp64"] = forms.pop("fp64_modal")
         line["other_forms"] = forms
         line["accuracy"] = accuracy

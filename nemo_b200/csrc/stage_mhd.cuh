@@ -361,10 +361,11 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
 // FP32 form: 3 CTAs per SM (168 registers, a few hundred bytes of spills; 2 % faster on B200 than
 // 4 CTAs at 128 registers with twice the spills, and 2 CTAs without spills is 14 % slower).  The update takes
 // nodes ab + 16 q of its element, coalesced rows of the register and the state (the x-line nodes, 32 bytes
-// apart, moved four sectors for one: 401 -> 336 us per stage at Orszag-Tang 32^3).  The conserved state is read per node pair
-// from the FP64 tile: a shared-memory array of per-node FP32 primitives (20 KB more per CTA) made the
-// pair fluxes cheaper but the stage 4 % slower, as the larger carveout left L1 too small for the
-// neighbour traces and register rows.
+// apart, moved four sectors for one: 401 -> 336 us per stage at Orszag-Tang 32^3).  The node pairs, faces and
+// subcells work on an FP32 copy of the tile made once (reading the FP64 tile they converted every node three
+// times over and conflicted four ways on the x-lines), whose place holds the rhs terms and subcell fluxes
+// afterwards: 57 KB of shared memory per CTA instead of 71, 336 -> 304 us.  What bounds it now is latency at 12
+// warps per SM: traces and rows from L2 (1.3 stalls per issue), dependent FP32 and MUFU chains (1.0, 0.8).
 template <typename R, bool BLEND, bool RHS_ONLY, bool FAST>
 __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArgs a) {
     constexpr int MEPC = mhd::EPC, MV = mhd::V;

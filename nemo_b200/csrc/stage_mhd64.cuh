@@ -12,7 +12,9 @@ namespace mhd64k {
 
 // Line form (a thread owned the three lines through (a, b): 255 registers, 8 warps per SM, every node's
 // primitives and divisions by mu0 recomputed per pair) -> this, B200, us per stage: Orszag-Tang 32^3
-// 1218 -> 636, 8^3 82 -> 23, 16^3 with Rusanov faces (general kernel) 187 -> 106.
+// 1218 -> 636, 8^3 82 -> 23, 16^3 with Rusanov faces (general kernel) 187 -> 106; with the neighbour ids read
+// ahead of the launch wait 611, 22, 104.  Bound by FP64 issue at 15 warps per SM (ncu, 32^3: issue 45 %, FP64
+// pipe 42 %; stalls per issue: dependent latency 1.9, loads 1.6, barriers 1.4).
 constexpr int MV = 9;
 constexpr int CTAS = 8;                          // resident elements per SM: 8 x 27 KB of shared memory,
                                                  // 128 registers
