@@ -1292,11 +1292,10 @@ int nemo_gpu_run_async(int64_t nsteps) {
     if (st) return st;
     if (nsteps <= 0) return fail(NEMO_ERR_ARG, "nsteps must be > 0");
     if (g.timing) return fail(NEMO_ERR_STATE, "timing mode runs synchronously (nemo_gpu_run)");
-    g.prepared = false;  // the CFL bound must belong to the current state
-    if ((st = prepare_if_needed())) return st;
-    // no end time (t_end = 0.0 is all-zero bits), not done
-    CK(cudaMemsetAsync(&g.ctrl->t_end, 0, sizeof(double), g.stream));
-    CK(cudaMemsetAsync(&g.ctrl->done, 0, sizeof(int32_t), g.stream));
+    // no end time, not done; the CFL bound must belong to the current state
+    CK(launch_ctrl_begin(g.ctrl, 0.0, g.stream));
+    CK(launch_prepare(true, g.stream));
+    g.prepared = true;
     for (int s = 0; s < 2; ++s)
         if (!g.graph[s] && (st = build_graph(s))) return st;
     for (int64_t i = 0; i < nsteps; ++i) {

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
     for (int r = 0; r < FETCH; ++r)
         nes[r] = (ND == 1 && r == 0) || tid + r * TPE < 6 * NF ? __ldg(a.nbr + e * 6 + 4 * r + (tid >> 4)) : -1;
     dep_sync();
-    if (!RHS_ONLY && ctrl->done) return;
+    if (!RHS_ONLY && !a.prep_only && ctrl->done) return;
     double* const su = smem + O_SU;
     double* const sp = smem + O_SP;
     double* const tr = smem + O_TR;
