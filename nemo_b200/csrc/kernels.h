@@ -11,9 +11,12 @@ namespace nemo {
 
 // Launch of a kernel of the step sequence (time step, mortars, stages): it may be set up while the kernel
 // before it in the stream drains, so that a launch costs no gap.  Such a kernel touches nothing another
-// kernel writes before its dep_sync().  us per stage in the step graphs without -> with it and with the
-// neighbour ids of the FP64 forms read ahead of the wait: GLM-MHD FP64 32^3 634 -> 611, 8^3 19.8 -> 19.4,
-// Euler FP64 4^3 15.7 -> 15.1, 16^3 45.8 -> 44.9, 32^3 380 -> 378; the FP32 forms 0.1-0.4 %.
+// kernel writes before its dep_sync(), and never reads such data through the read-only path (__ldg), which
+// asks for data that nobody writes while the kernel lives: its life begins before the writer's ends.  The
+// read-only path is for the mesh tables (nbr, cdel), which no kernel writes.
+// us per stage in the step graphs without -> with it and with the neighbour ids of the FP64 forms read ahead
+// of the wait: GLM-MHD FP64 32^3 634 -> 611, 8^3 19.8 -> 19.4, Euler FP64 4^3 15.7 -> 15.1, 16^3 45.8 -> 44.9,
+// 32^3 380 -> 378; the FP32 forms 0.1-0.4 %.
 template <typename... KArgs>
 inline cudaError_t launch_dep(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
                               KArgs... args) {

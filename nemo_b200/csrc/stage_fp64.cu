@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
     for (int r = 0; r < FETCH; ++r)
         nes[r] = (ND == 1 && r == 0) || tid + r * TPE < 6 * NF ? __ldg(a.nbr + e * 6 + 4 * r + (tid >> 4)) : -1;
     dep_sync();
-    if (!RHS_ONLY && !a.prep_only && ctrl->done) return;
+    if (!RHS_ONLY && ctrl->done && !a.prep_only) return;
     double* const su = smem + O_SU;
     double* const sp = smem + O_SP;
     double* const tr = smem + O_TR;
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
 
     double q[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
+    for (int v = 0; v < V; ++v) q[v] = __ldcg(a.u_in + ((int64_t)v * E + e) * NP + n);
     auto epilogue = [&]() {
         epilogue64<ND>(a, q[0], pressure64(q, k), sp, s_vi, s_lam, e, n, k, [&](int dd) {
             const double rr[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(TPE, mhd64k::CTAS) k_stage_mhd64(StageArgs a) 
 
     double q[MV];
 #pragma unroll
-    for (int v = 0; v < MV; ++v) q[v] = __ldg(a.u_in + ((int64_t)v * E + e) * NP + n);
+    for (int v = 0; v < MV; ++v) q[v] = __ldcg(a.u_in + ((int64_t)v * E + e) * NP + n);
     auto epilogue = [&]() {
         epilogue64<1>(a, q[0], m_pressure<double>(q, k.kappa, FAST ? 1.0 : k.mu0), sp, s_vi, s_lam, e, n, k,
                    [&](int dd) {
