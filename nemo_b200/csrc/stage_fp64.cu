@@ -226,6 +226,7 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
                     const double x = f / 10.0 + 1.0;
                     if (x < a.mlp64[MLP_NW + lane] || x > a.mlp64[MLP_NW + 12 + lane]) fb = 1;
                 }
+                __syncwarp();   // feat[]: a vote orders no memory
                 fb = __any_sync(0xffffffffu, fb);
                 const double* W1 = a.mlp64;
                 const double* b1 = W1 + 32 * 12;

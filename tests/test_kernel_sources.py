@@ -35,3 +35,12 @@ def test_dependent_launches_read_written_data_by_ordinary_loads():
             for arg in re.findall(r"__ldg\(\s*&?([\w.\->]+)", body):
                 assert arg in MESH_TABLES, (head, arg)
     assert seen == deps
+
+
+def test_features_are_ordered_before_the_first_layer():
+    """The learned indicator's features pass between the lanes of a warp through shared memory: a barrier that
+    orders memory (a vote does not) stands between the writes and the reads."""
+    text = open(os.path.join(CSRC, "stage_fp64.cu")).read()
+    body, = [b for h, b in functions(text) if "epilogue64(" in h]
+    between = body[body.index("feat[lane] = "):body.index("feat[i]")]
+    assert "__syncwarp();" in between
