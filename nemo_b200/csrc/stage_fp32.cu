@@ -286,7 +286,6 @@ __device__ __forceinline__ void epilogue32(const StageArgs& a, const double* su,
     __shared__ float s_jd[EPC];
     __shared__ double s_dt[EPC], s_lm[EPC];
     __shared__ int s_gr[EPC];
-    if (threadIdx.x < EPC) s_fb[threadIdx.x] = 0;
     // the thread reads nodes ab + 16 i of the FP64 state (no bank conflicts) and hands rho and p on
     // through the scratch to the threads of their x-lines
     float qr[NN], qp[NN];
@@ -470,12 +469,10 @@ __device__ __forceinline__ void epilogue32(const StageArgs& a, const double* su,
             const float z = hsum16(W3[j0] * g0 + W3[j0 + 1] * g1) + W3[32];
             float al = k.alpha_max32 / (1.0f + __expf(-z));
             if (al < k.alpha_min32) al = 0.0f;
-            if (fb) {
-                alpha = am;
-                if (active && ab == 0) s_fb[el] = 1;
-            } else {
-                alpha = al;
-                if (active && ab == 0) s_jd[el] = fabsf(al - am);
+            alpha = fb ? am : al;
+            if (active && ab == 0) {
+                s_fb[el] = fb;
+                s_jd[el] = fabsf(al - am);
             }
         }
         if (active && ab == 0) a.alpha_out[e] = (double)alpha;

@@ -44,3 +44,11 @@ def test_features_are_ordered_before_the_first_layer():
     body, = [b for h, b in functions(text) if "epilogue64(" in h]
     between = body[body.index("feat[lane] = "):body.index("feat[i]")]
     assert "__syncwarp();" in between
+
+
+def test_fallback_flag_is_written_by_its_own_element():
+    """FP32 form: the flag of an element is set either way by a thread of that element, not cleared by a thread of
+    another warp without a barrier before it is set."""
+    text = open(os.path.join(CSRC, "stage_fp32.cu")).read()
+    body, = [b for h, b in functions(text) if "epilogue32(" in h]
+    assert re.findall(r"s_fb\[(.*?)\] =", body) == ["el"]
