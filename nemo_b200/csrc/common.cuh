@@ -77,6 +77,7 @@ struct OpConsts {
     double repair_decr;
     double mu0;
     double skm1;           // 1/(kappa-1)
+    int quick;             // kappa and mu0 leave the flux quotients inside the domain of ieee64.cuh
     int cool;              // barotropic cooling after every stage
     double cool_rho;       // dens_critical
     double cool_ci;        // k_isothermal / (kappa - 1)

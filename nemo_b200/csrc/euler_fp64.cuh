@@ -26,8 +26,9 @@ __device__ __forceinline__ double xlambda64(const double* u, const OpConsts& k) 
 
 // pressure, and xflux (source/equations/euler/equations_mod.f90:64-79), with the reciprocal of the
 // density at hand (flux kernels)
+template <class A>
 __device__ __forceinline__ double pressure64(const double* u, const Rcp64& r, const OpConsts& k) {
-    return k.km1 * (u[4] - quot64(0.5, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]));
+    return k.km1 * (u[4] - A::quot(0.5, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]));
 }
 
 __device__ __forceinline__ void xflux64(const double* u, double velx, double pres, double* f) {
@@ -40,23 +41,24 @@ __device__ __forceinline__ void xflux64(const double* u, double velx, double pre
 
 // HLLC/HLLE hybrid, source/equations/euler/riemann/hllc/riemann_mod.f90:7-104.  Nine of its quotients
 // share a density, two the sum of the roots and five the width of the fan.
+template <class A>
 __device__ __forceinline__ void hllc64(const double* UL, const double* UR, double* F, const OpConsts& k) {
     const double kappa = k.kappa;
     const double beta = k.hllc_beta;
-    const Rcp64 rL = rcp64r(UL[0]), rR = rcp64r(UR[0]);
-    double VL = quot64(UL[1], rL);
-    double VR = quot64(UR[1], rR);
-    double pL = pressure64(UL, rL, k);
-    double pR = pressure64(UR, rR, k);
-    double cL = sqrt64(quot64(kappa * pL, rL));
-    double cR = sqrt64(quot64(kappa * pR, rR));
-    double HL = quot64(UL[4] + pL, rL);
-    double HR = quot64(UR[4] + pR, rR);
-    double sL = sqrt64(UL[0]), sR = sqrt64(UR[0]);
-    const Rcp64 rs = rcp64r(sL + sR);
-    double Ht = quot64(sL * HL + sR * HR, rs);
-    double vt = quot64(sL * VL + sR * VR, rs);
-    double at = sqrt64(k.km1 * (Ht - 0.5 * (vt * vt)));
+    const Rcp64 rL = A::rcp(UL[0]), rR = A::rcp(UR[0]);
+    double VL = A::quot(UL[1], rL);
+    double VR = A::quot(UR[1], rR);
+    double pL = pressure64<A>(UL, rL, k);
+    double pR = pressure64<A>(UR, rR, k);
+    double cL = A::root(A::quot(kappa * pL, rL));
+    double cR = A::root(A::quot(kappa * pR, rR));
+    double HL = A::quot(UL[4] + pL, rL);
+    double HR = A::quot(UR[4] + pR, rR);
+    double sL = A::root(UL[0]), sR = A::root(UR[0]);
+    const Rcp64 rs = A::rcp(sL + sR);
+    double Ht = A::quot(sL * HL + sR * HR, rs);
+    double vt = A::quot(sL * VL + sR * VR, rs);
+    double at = A::root(k.km1 * (Ht - 0.5 * (vt * vt)));
     double SL = fmin(fmin(vt - at, VL - beta * cL), 0.0);
     double SR = fmax(fmax(vt + at, VR + beta * cR), 0.0);
     // the supersonic cases (SL >= 0: the left flux, SR <= 0: the right flux) are selected at the
@@ -66,8 +68,8 @@ __device__ __forceinline__ void hllc64(const double* UL, const double* UR, doubl
     xflux64(UL, VL, pL, FL);
     xflux64(UR, VR, pR, FR);
     const bool supL = SL >= 0.0, supR = SR <= 0.0;
-    double smooth = sqrt64(div64(fabs(pL - pR), pL + pR));
-    double SS = div64(pR - pL + UL[1] * (SL - VL) - UR[1] * (SR - VR), UL[0] * (SL - VL) - UR[0] * (SR - VR));
+    double smooth = A::root(A::div(fabs(pL - pR), pL + pR));
+    double SS = A::div(pR - pL + UL[1] * (SL - VL) - UR[1] * (SR - VR), UL[0] * (SL - VL) - UR[0] * (SR - VR));
     const bool left = (SL <= 0.0 && 0.0 <= SS);
     double U[5], FU[5];
 #pragma unroll
@@ -79,51 +81,45 @@ __device__ __forceinline__ void hllc64(const double* UL, const double* UR, doubl
     const double S = left ? SL : SR;
     const double V = left ? VL : VR;
     const double p = left ? pL : pR;
-    double Q = div64(U[0] * (S - V), S - SS);
+    double Q = A::div(U[0] * (S - V), S - SS);
     double Us[5];
     Us[0] = Q;
     Us[1] = Q * SS;
-    Us[2] = quot64(Q * U[2], rU);
-    Us[3] = quot64(Q * U[3], rU);
-    Us[4] = Q * (quot64(U[4], rU) + (SS - V) * (SS + div64(quot64(p, rU), S - V)));
+    Us[2] = A::quot(Q * U[2], rU);
+    Us[3] = A::quot(Q * U[3], rU);
+    Us[4] = Q * (A::quot(U[4], rU) + (SS - V) * (SS + A::div(A::quot(p, rU), S - V)));
     const double oms = 1.0 - smooth;
     const double SLSR = SL * SR;
-    const Rcp64 rd = rcp64r(SR - SL);
+    const Rcp64 rd = A::rcp(SR - SL);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        double FH = quot64(SR * FL[v] - SL * FR[v] + SLSR * (UR[v] - UL[v]), rd);
+        double FH = A::quot(SR * FL[v] - SL * FR[v] + SLSR * (UR[v] - UL[v]), rd);
         const double Fm = smooth * FH + oms * (FU[v] + S * (Us[v] - U[v]));
         F[v] = supL ? FL[v] : (supR ? FR[v] : Fm);
     }
 }
 
 // Rusanov, source/equations/euler/riemann/rusanov/riemann_mod.f90:7-24
+template <class A>
 __device__ __forceinline__ void rusanov64(const double* uL, const double* uR, double* F, const OpConsts& k) {
     double FL[5], FR[5];
-    const Rcp64 rL = rcp64r(uL[0]), rR = rcp64r(uR[0]);
-    const double VL = quot64(uL[1], rL), VR = quot64(uR[1], rR);
-    double pL = pressure64(uL, rL, k), pR = pressure64(uR, rR, k);
+    const Rcp64 rL = A::rcp(uL[0]), rR = A::rcp(uR[0]);
+    const double VL = A::quot(uL[1], rL), VR = A::quot(uR[1], rR);
+    double pL = pressure64<A>(uL, rL, k), pR = pressure64<A>(uR, rR, k);
     xflux64(uL, VL, pL, FL);
     xflux64(uR, VR, pR, FR);
-    double lL = fabs(VL) + sqrt64(quot64(k.kappa * pL, rL));
-    double lR = fabs(VR) + sqrt64(quot64(k.kappa * pR, rR));
+    double lL = fabs(VL) + A::root(A::quot(k.kappa * pL, rL));
+    double lR = fabs(VR) + A::root(A::quot(k.kappa * pR, rR));
     double lmax = fmax(lL, lR);
 #pragma unroll
     for (int v = 0; v < 5; ++v) F[v] = 0.5 * (FL[v] + FR[v] + lmax * (uL[v] - uR[v]));
 }
 
-__device__ __forceinline__ void riemann64(int kind, const double* uL, const double* uR, double* F,
-                                          const OpConsts& k) {
-    if (kind == 1) rusanov64(uL, uR, F, k);
-    else hllc64(uL, uR, F, k);
-}
-
-// FAST: the flux kinds fixed at compile time (HLLC faces and subcells, Chandrashekar pairs); a
-// run-time switch inside the unrolled line loops is a branch around every flux
-template <bool FAST>
+// FAST: HLLC fixed at compile time (a run-time switch is a branch around every flux)
+template <class A, bool FAST>
 __device__ __forceinline__ void riem64(int kind, const double* uL, const double* uR, double* F, const OpConsts& k) {
-    if (FAST) hllc64(uL, uR, F, k);
-    else riemann64(kind, uL, uR, F, k);
+    if (!FAST && kind == 1) rusanov64<A>(uL, uR, F, k);
+    else hllc64<A>(uL, uR, F, k);
 }
 
 // logmean with the absolute switch, source/equations/euler/two_point/chandrashekar/
@@ -132,12 +128,13 @@ __device__ __forceinline__ void riem64(int kind, const double* uL, const double*
 // per stage at Sedov 32^3, 48.1 against 49.1 us on the smooth wave at 16^3.)
 static __constant__ double LM_C[4] = {1e-4, 1.0 / 6.0, 2.0 / 45.0, 22.0 / 945.0};
 
+template <class A>
 __device__ __forceinline__ double logmean64(double a, double b, double x) {
     if (fabs(a - b) < LM_C[0]) {
-        const double u = div64(x * (x - 2.0) + 1.0, x * (x + 2.0) + 1.0);
+        const double u = A::div(x * (x - 2.0) + 1.0, x * (x + 2.0) + 1.0);
         return (a + b) * (0.5 - u * (LM_C[1] - u * (LM_C[2] - LM_C[3] * u)));
     }
-    return div64(a - b, plog64(x));
+    return A::div(a - b, plog64(x));
 }
 
 // Per-node primitive data of the two-point flux: rho and its reciprocal, normal/tangential velocities,
@@ -148,15 +145,16 @@ struct Node5 {
 
 // Chandrashekar EC/KEP flux, two_point_flux_mod.f90:34-77 (the per-node quantities pressure,
 // beta = 0.5*rho/p and velocities are computed once per node with the same expressions).
+template <class A>
 __device__ __forceinline__ void chandrashekar64(const Node5& u, const Node5& v, double* f, const OpConsts& k) {
-    const double dens = logmean64(u.rho, v.rho, quot64(u.rho, Rcp64{v.rho, v.y}));
+    const double dens = logmean64<A>(u.rho, v.rho, A::quot(u.rho, Rcp64{v.rho, v.y}));
     double velx = 0.5 * (u.vn + v.vn);
     double vely = 0.5 * (u.vt1 + v.vt1);
     double velz = 0.5 * (u.vt2 + v.vt2);
-    double pres = div64(0.5 * (u.rho + v.rho), u.beta + v.beta);
+    double pres = A::div(0.5 * (u.rho + v.rho), u.beta + v.beta);
     double ssum = (u.vn * u.vn + v.vn * v.vn) + (u.vt1 * u.vt1 + v.vt1 * v.vt1);
     ssum = ssum + (u.vt2 * u.vt2 + v.vt2 * v.vt2);
-    double enth = div64(k.c_enth, logmean64(u.beta, v.beta, div64(u.beta, v.beta))) + div64(pres, dens) + velx * velx +
+    double enth = A::div(k.c_enth, logmean64<A>(u.beta, v.beta, A::div(u.beta, v.beta))) + A::div(pres, dens) + velx * velx +
                   vely * vely + velz * velz - 0.25 * ssum;
     f[0] = dens * velx;
     f[1] = f[0] * velx + pres;
@@ -166,13 +164,33 @@ __device__ __forceinline__ void chandrashekar64(const Node5& u, const Node5& v, 
 }
 
 // central flux 0.5*(f(u)+f(v)), source/equations/euler/two_point/standard/two_point_flux_mod.f90:13-49
+template <class A>
 __device__ __forceinline__ void central64(const double* u, const double* v, double* f, const OpConsts& k) {
     double fu[5], fv[5];
-    const Rcp64 ru = rcp64r(u[0]), rv = rcp64r(v[0]);
-    xflux64(u, quot64(u[1], ru), pressure64(u, ru, k), fu);
-    xflux64(v, quot64(v[1], rv), pressure64(v, rv, k), fv);
+    const Rcp64 ru = A::rcp(u[0]), rv = A::rcp(v[0]);
+    xflux64(u, A::quot(u[1], ru), pressure64<A>(u, ru, k), fu);
+    xflux64(v, A::quot(v[1], rv), pressure64<A>(v, rv, k), fv);
 #pragma unroll
     for (int c = 0; c < 5; ++c) f[c] = 0.5 * (fu[c] + fv[c]);
+}
+
+// Whether every flux of this state against another such state keeps Quick64's operands inside its domain:
+// density and energy within 2^+-100, internal at least 2^-30 of total energy (velocities up to 2^20 sound
+// speeds), no momentum between 0 and 2^-280.  With kappa - 1 within 2^-10..2^10 the pressure is then at least
+// 2^-140, no speed of the fan nor what is left of a cancelling sum of them lies between 0 and 2^-179, the smallest
+// numerator (the product of two momenta in the mean over the fan) is 2^-891 and the smallest quotient 2^-997.
+// Ordinary flows meet the last condition: in a still ambient the exponents of the momenta double with every few
+// elements from the disturbance (2^-229 on Sedov 32^3 after 40 steps).  A NaN fails the comparisons.
+__device__ __forceinline__ bool within64(double x, int e) {   // 2^-e <= x < 2^e
+    return (unsigned)__double2hiint(x) - ((1023u - e) << 20) < (unsigned)(2 * e) << 20;
+}
+__device__ __forceinline__ bool tiny64(double x, double limit) { return fabs(x) < limit && x != 0.0; }
+
+__device__ __forceinline__ bool regular64(const double* u) {
+    const double re = u[0] * u[4];
+    const double ri = fma(-0.5, fma(u[1], u[1], fma(u[2], u[2], u[3] * u[3])), re);
+    return within64(u[0], 100) && within64(u[4], 100) && ri >= 0x1p-30 * re && !tiny64(u[1], 0x1p-280) &&
+           !tiny64(u[2], 0x1p-280) && !tiny64(u[3], 0x1p-280);
 }
 
 __device__ __forceinline__ bool isvalid64(const double* u, const OpConsts& k) {

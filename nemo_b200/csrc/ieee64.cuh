@@ -15,9 +15,11 @@
 // is the same idea on y ~ 1/sqrt(a): g = RN(a y), RN(g + (a - g^2) y/2).
 //
 // Domain: operands, results and their products with a few ulp's worth of residual in the normal range
-// (|a| above about 1e-290).  A zero quotient comes back as +0; a zero, infinite or NaN denominator gives
-// NaN, as does an infinite numerator.  Same bits as / and sqrt otherwise (checked against them on 1.9e9
-// pairs chosen next to a tie, 5e8 random ones and all pairs within 2000 ulp of 1 and 2, and by every bit-exact test of the plain path).
+// (|a| zero or above about 1e-290, |b| from 2^-1000 to 2^1000); the square root's argument likewise.  A zero
+// quotient comes back as +0.  Outside, a last bit is lost, a zero or infinite denominator and an infinite numerator
+// give NaN: callers see to it that no operand is (regular64 in euler_fp64.cuh), or take Plain64.  Same bits as /
+// and sqrt inside (tests/test_gpu_fp64_domain.py: quotients next to a rounding tie, significands of all ones,
+// the neighbourhoods of powers of two, random operands over the whole domain).
 // What they give: the stage kernel of stage_fp64.cu, Sedov 32^3, 727 us with / and sqrt (340 M warp
 // instructions), 381 us with these and 24 warps per SM (242 M).
 #pragma once
@@ -55,5 +57,20 @@ __device__ __forceinline__ double sqrt64(double a) {
     const double s = fma(fma(-g, g, a), 0.5 * y, g);
     return a == 0.0 ? a : s;
 }
+
+// The two arithmetics of a flux: the quotients above, for operands inside their domain, and the language's own
+// for any operands.
+struct Quick64 {
+    static __device__ __forceinline__ Rcp64 rcp(double b) { return rcp64r(b); }
+    static __device__ __forceinline__ double quot(double a, const Rcp64& r) { return quot64(a, r); }
+    static __device__ __forceinline__ double div(double a, double b) { return div64(a, b); }
+    static __device__ __forceinline__ double root(double a) { return sqrt64(a); }
+};
+struct Plain64 {
+    static __device__ __forceinline__ Rcp64 rcp(double b) { return {b, 0.0}; }
+    static __device__ __forceinline__ double quot(double a, const Rcp64& r) { return a / r.b; }
+    static __device__ __forceinline__ double div(double a, double b) { return a / b; }
+    static __device__ __forceinline__ double root(double a) { return sqrt(a); }
+};
 
 }  // namespace nemo

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "euler_fp64.cuh"
 #include "ieee64.cuh"
 #include "mhd_phys.cuh"
 #include "pmath64.cuh"
@@ -27,20 +28,20 @@ __device__ __forceinline__ Mhd64<MU1> mhd64(const OpConsts& k, double ch) {
 }
 
 // pressure_elemental, source/equations/mhd/equations_mod.f90:223-234, with the reciprocal of the density
-template <bool MU1>
+template <class A, bool MU1>
 __device__ __forceinline__ double m_pressure64(const double* u, const Rcp64& r, const Mhd64<MU1>& P) {
     const double h = MU1 ? 0.5 : 0.5 / P.mu0_;
-    return P.km1 * (u[4] - quot64(0.5, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) -
+    return P.km1 * (u[4] - A::quot(0.5, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) -
                     h * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7] + u[8] * u[8]));
 }
 
 // xflux, equations_mod.f90:64-139
-template <bool MU1>
+template <class A, bool MU1>
 __device__ __forceinline__ void m_xflux64(const double* U, const Rcp64& r, double* f, const Mhd64<MU1>& P) {
     const double kappaM2 = P.kappa - 2.0, s2mu_0 = MU1 ? 0.5 : 0.5 / P.mu0_;
     const double hmu = MU1 ? 0.5 : 0.5 * (1.0 / P.mu0_);
     const double Etotal = U[4] - hmu * (U[8] * U[8]);
-    const double srho = quot64(1.0, r);
+    const double srho = A::quot(1.0, r);
     const double v1 = U[1] * srho, v2 = U[2] * srho, v3 = U[3] * srho;
     const double v_2 = v1 * v1 + v2 * v2 + v3 * v3;
     const double bb2 = U[5] * U[5] + U[6] * U[6] + U[7] * U[7];
@@ -62,30 +63,31 @@ __device__ __forceinline__ void m_xflux64(const double* U, const Rcp64& r, doubl
 }
 
 // Fastest_Signal_Speed + xlambdaMax, equations_mod.f90:693-714, :522-531
-template <bool MU1>
+template <class A, bool MU1>
 __device__ __forceinline__ double m_xlambda64(const double* U, const Rcp64& r, const Mhd64<MU1>& P) {
-    const double pres = m_pressure64(U, r, P);
-    const double cs2 = quot64(P.kappa * pres, r);
-    const double ca2 = P.over_mu(quot64(U[5] * U[5], r));
-    const double va2 = P.over_mu(quot64(U[6] * U[6] + U[7] * U[7], r)) + ca2;
-    const double astar = sqrt64((cs2 + va2) * (cs2 + va2) - 4.0 * cs2 * ca2);
-    const double c = sqrt64(0.5 * (cs2 + va2 + astar));
-    return fabs(quot64(U[1], r)) + c;
+    const double pres = m_pressure64<A>(U, r, P);
+    const double cs2 = A::quot(P.kappa * pres, r);
+    const double ca2 = P.over_mu(A::quot(U[5] * U[5], r));
+    const double va2 = P.over_mu(A::quot(U[6] * U[6] + U[7] * U[7], r)) + ca2;
+    const double astar = A::root((cs2 + va2) * (cs2 + va2) - 4.0 * cs2 * ca2);
+    const double c = A::root(0.5 * (cs2 + va2 + astar));
+    return fabs(A::quot(U[1], r)) + c;
 }
 
 // Rusanov, source/equations/mhd/riemann/rusanov/riemann_mod.f90:7-24
-template <bool MU1>
+template <class A, bool MU1>
 __device__ __forceinline__ void m_rusanov64(const double* uL, const double* uR, double* F, const Mhd64<MU1>& P) {
     double FL[9], FR[9];
-    const Rcp64 rL = rcp64r(uL[0]), rR = rcp64r(uR[0]);
-    m_xflux64(uL, rL, FL, P);
-    m_xflux64(uR, rR, FR, P);
-    const double lmax = fmax(m_xlambda64(uL, rL, P), m_xlambda64(uR, rR, P));
+    const Rcp64 rL = A::rcp(uL[0]), rR = A::rcp(uR[0]);
+    m_xflux64<A>(uL, rL, FL, P);
+    m_xflux64<A>(uR, rR, FR, P);
+    const double lmax = fmax(m_xlambda64<A>(uL, rL, P), m_xlambda64<A>(uR, rR, P));
 #pragma unroll
     for (int v = 0; v < 9; ++v) F[v] = 0.5 * (FL[v] + FR[v] + lmax * (uL[v] - uR[v]));
 }
 
 // HLLD with the GLM pair upwind, as m_hlld_x (mhd_phys.cuh) expression by expression
+template <class A>
 __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, double* F, const Mhd64<true>& P) {
     const double half = 0.5, kappa = P.kappa;
     const Rcp64 rkm1 = {P.km1, P.skm1};
@@ -96,22 +98,22 @@ __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, dou
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const double* u = s ? uR : uL;
-        const Rcp64 r = rcp64r(u[0]);
+        const Rcp64 r = A::rcp(u[0]);
         rho[s] = u[0];
-        un[s] = quot64(u[1], r);
-        vt1[s] = quot64(u[2], r);
-        vt2[s] = quot64(u[3], r);
+        un[s] = A::quot(u[1], r);
+        vt1[s] = A::quot(u[2], r);
+        vt2[s] = A::quot(u[3], r);
         bt1[s] = u[6];
         bt2[s] = u[7];
-        const double pr = P.km1 * (u[4] - quot64(half, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) -
+        const double pr = P.km1 * (u[4] - A::quot(half, r) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) -
                                    half * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7] + u[8] * u[8]));
         const double bb = bn2 + bt1[s] * bt1[s] + bt2[s] * bt2[s];
-        et[s] = quot64(pr, rkm1) + half * rho[s] * (un[s] * un[s] + vt1[s] * vt1[s] + vt2[s] * vt2[s]) + half * bb;
+        et[s] = A::quot(pr, rkm1) + half * rho[s] * (un[s] * un[s] + vt1[s] * vt1[s] + vt2[s] * vt2[s]) + half * bb;
         pt[s] = pr + half * bb;
-        const double cs2 = quot64(kappa * pr, r);
-        const double ca2 = quot64(bn2, r);
-        const double va2 = quot64(bb, r);
-        cf[s] = sqrt64(half * (cs2 + va2 + sqrt64((cs2 + va2) * (cs2 + va2) - 4.0 * cs2 * ca2)));
+        const double cs2 = A::quot(kappa * pr, r);
+        const double ca2 = A::quot(bn2, r);
+        const double va2 = A::quot(bb, r);
+        cf[s] = A::root(half * (cs2 + va2 + A::root((cs2 + va2) * (cs2 + va2) - 4.0 * cs2 * ca2)));
     }
     const double cmax = fmax(cf[0], cf[1]);
     const double SL = fmin(un[0], un[1]) - cmax;
@@ -146,19 +148,19 @@ __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, dou
         for (int v = 0; v < 8; ++v) F[v] = Fk[1][v];
     } else {
         const double dL = rho[0] * (SL - un[0]), dR = rho[1] * (SR - un[1]);
-        const double SM = div64(dR * un[1] - dL * un[0] - pt[1] + pt[0], dR - dL);
+        const double SM = A::div(dR * un[1] - dL * un[0] - pt[1] + pt[0], dR - dL);
         const double ptS = pt[0] + dL * (SM - un[0]);
         double rs[2], ws1[2], ws2[2], cs1[2], cs2[2], es[2];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const double S = s ? SR : SL;
             const double d = s ? dR : dL;
-            const Rcp64 rS = rcp64r(S - SM);
-            rs[s] = quot64(d, rS);
+            const Rcp64 rS = A::rcp(S - SM);
+            rs[s] = A::quot(d, rS);
             const double den = d * (S - SM) - bn2;
-            const Rcp64 rden = rcp64r(den);
-            const double fv = quot64(bn * (SM - un[s]), rden);
-            const double fb = quot64(d * (S - un[s]) - bn2, rden);
+            const Rcp64 rden = A::rcp(den);
+            const double fv = A::quot(bn * (SM - un[s]), rden);
+            const double fb = A::quot(d * (S - un[s]) - bn2, rden);
             const bool flat = fabs(den) < 1.0e-8;
             ws1[s] = flat ? vt1[s] : vt1[s] - fv * bt1[s];
             ws2[s] = flat ? vt2[s] : vt2[s] - fv * bt2[s];
@@ -166,10 +168,10 @@ __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, dou
             cs2[s] = flat ? bt2[s] : fb * bt2[s];
             const double vb = un[s] * bn + vt1[s] * bt1[s] + vt2[s] * bt2[s];
             const double vbs = SM * bn + ws1[s] * cs1[s] + ws2[s] * cs2[s];
-            es[s] = quot64((S - un[s]) * et[s] - pt[s] * un[s] + ptS * SM + bn * (vb - vbs), rS);
+            es[s] = A::quot((S - un[s]) * et[s] - pt[s] * un[s] + ptS * SM + bn * (vb - vbs), rS);
         }
-        const double sqL = sqrt64(rs[0]), sqR = sqrt64(rs[1]);
-        const double SLs = SM - div64(fabs(bn), sqL), SRs = SM + div64(fabs(bn), sqR);
+        const double sqL = A::root(rs[0]), sqR = A::root(rs[1]);
+        const double SLs = SM - A::div(fabs(bn), sqL), SRs = SM + A::div(fabs(bn), sqR);
         const bool sr = !(SM >= 0.0);
         const double S = sr ? SR : SL;
         const double rsS = sr ? rs[1] : rs[0], ws1S = sr ? ws1[1] : ws1[0], ws2S = sr ? ws2[1] : ws2[0];
@@ -188,7 +190,7 @@ __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, dou
             for (int v = 0; v < 8; ++v) Uss[v] = Us[v];
             if (fabs(bn) >= 1.0e-12) {
                 const double sg = bn < 0.0 ? -1.0 : 1.0;
-                const double sden = div64(1.0, sqL + sqR);
+                const double sden = A::div(1.0, sqL + sqR);
                 const double w1 = (sqL * ws1[0] + sqR * ws1[1] + sg * (cs1[1] - cs1[0])) * sden;
                 const double w2 = (sqL * ws2[0] + sqR * ws2[1] + sg * (cs2[1] - cs2[0])) * sden;
                 const double c1 = (sqL * cs1[1] + sqR * cs1[0] + sg * sqL * sqR * (ws1[1] - ws1[0])) * sden;
@@ -218,10 +220,11 @@ __device__ __forceinline__ void m_hlld64(const double* uL, const double* uR, dou
 // LN_MEAN, source/equations/mhd/two_point/ec/two_point_flux_mod.f90:203-219 (relative switch); Xi = aR/aL
 static __constant__ double LNM_EPS = 1.0e-4;
 
+template <class A>
 __device__ __forceinline__ double ln_mean64(double aL, double aR, double Xi) {
-    const double u = div64(Xi * (Xi - 2.0) + 1.0, Xi * (Xi + 2.0) + 1.0);
-    if (u < LNM_EPS) return div64((aL + aR) * 52.5, 105.0 + u * (35.0 + u * (21.0 + u * 15.0)));
-    return div64(aR - aL, plog64(Xi));
+    const double u = A::div(Xi * (Xi - 2.0) + 1.0, Xi * (Xi + 2.0) + 1.0);
+    if (u < LNM_EPS) return A::div((aL + aR) * 52.5, 105.0 + u * (35.0 + u * (21.0 + u * 15.0)));
+    return A::div(aR - aL, plog64(Xi));
 }
 
 // Per-node data of the two-point flux in the frame of a direction
@@ -229,29 +232,29 @@ struct MNode64 {
     double rho, y, v[3], B[3], psi, beta;   // y = 1/rho, beta = rho/(2 p) with p in that frame's order
 };
 
-// beta of the EC flux (its pressure subtracts psi^2/2 first), momentum and field in the frame's order
+// pressure of the EC flux, whose beta is rho/(2 p) (psi^2/2 is subtracted first), momentum and field in the
+// frame's order
 template <bool MU1>
-__device__ __forceinline__ double m_beta64(double rho, const double* v, const double* B, double E, double psi,
-                                           const Mhd64<MU1>& P) {
+__device__ __forceinline__ double m_p64(double rho, const double* v, const double* B, double E, double psi,
+                                        const Mhd64<MU1>& P) {
     const double hmu = MU1 ? 0.5 : 0.5 * (1.0 / P.mu0_);
     const double E1 = E - hmu * (psi * psi);
     const double v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
     const double B2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
-    const double p = P.km1 * (E1 - 0.5 * (rho * v2 + P.smu(B2)));
-    return div64(0.5 * rho, p);
+    return P.km1 * (E1 - 0.5 * (rho * v2 + P.smu(B2)));
 }
 
 // EC (Derigs) flux, source/equations/mhd/two_point/ec/two_point_flux_mod.f90:13-86.  In the places of
 // F[5] and F[8] it returns {psi} and {B_n}, from which the gathering node forms both (c_h {psi}, c_h {B_n})
 // and its non-conservative term.
-template <bool MU1>
+template <class A, bool MU1>
 __device__ __forceinline__ void m_ec64(const MNode64& L, const MNode64& R, double* F, const Mhd64<MU1>& P) {
     const double v2_L = L.v[0] * L.v[0] + L.v[1] * L.v[1] + L.v[2] * L.v[2];
     const double v2_R = R.v[0] * R.v[0] + R.v[1] * R.v[1] + R.v[2] * R.v[2];
     const double B2_L = L.B[0] * L.B[0] + L.B[1] * L.B[1] + L.B[2] * L.B[2];
     const double B2_R = R.B[0] * R.B[0] + R.B[1] * R.B[1] + R.B[2] * R.B[2];
-    const double rhoLN = ln_mean64(L.rho, R.rho, quot64(R.rho, Rcp64{L.rho, L.y}));
-    const double betaLN = ln_mean64(L.beta, R.beta, div64(R.beta, L.beta));
+    const double rhoLN = ln_mean64<A>(L.rho, R.rho, A::quot(R.rho, Rcp64{L.rho, L.y}));
+    const double betaLN = ln_mean64<A>(L.beta, R.beta, A::div(R.beta, L.beta));
     double vAvg[3], BAvg[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -262,7 +265,7 @@ __device__ __forceinline__ void m_ec64(const MNode64& L, const MNode64& R, doubl
     const double vB_Avg = 0.5 * ((L.v[0] * L.B[0] + L.v[1] * L.B[1] + L.v[2] * L.B[2]) +
                                  (R.v[0] * R.B[0] + R.v[1] * R.B[1] + R.v[2] * R.B[2]));
     const double hs = MU1 ? 0.5 : (1.0 / P.mu0_) * 0.5;
-    const double pTilde = 0.5 * (div64(L.rho + R.rho, L.beta + R.beta) + hs * (B2_L + B2_R));
+    const double pTilde = 0.5 * (A::div(L.rho + R.rho, L.beta + R.beta) + hs * (B2_L + B2_R));
     const double psiAvg = 0.5 * (L.psi + R.psi);
     const double sB = P.smu(BAvg[0]);
     F[0] = rhoLN * vAvg[0];
@@ -274,7 +277,7 @@ __device__ __forceinline__ void m_ec64(const MNode64& L, const MNode64& R, doubl
     const double F5 = P.ch * psiAvg, F8 = P.ch * BAvg[0];
     const double s1 = vAvg[0] * F[1] + vAvg[1] * F[2] + vAvg[2] * F[3];
     const double s2 = BAvg[0] * F5 + BAvg[1] * F[6] + BAvg[2] * F[7];
-    F[4] = F[0] * 0.5 * (div64(P.skm1, betaLN) - 0.5 * (v2_L + v2_R)) + s1 +
+    F[4] = F[0] * 0.5 * (A::div(P.skm1, betaLN) - 0.5 * (v2_L + v2_R)) + s1 +
            P.smu(s2 - 0.5 * v1_B2Avg + BAvg[0] * vB_Avg + F8 * psiAvg - P.ch * 0.5 * (L.psi * L.B[0] + R.psi * R.B[0]));
     F[5] = psiAvg;
     F[8] = BAvg[0];
@@ -294,6 +297,22 @@ __device__ __forceinline__ void m_add_nc64(double* F, const double* v, const dou
     }
     F[4] = F[4] + (P.over_mu(Bavg * vB) + gv * P.over_mu(psi));
     F[8] = F[8] + gv;
+}
+
+// As regular64 (euler_fp64.cuh): density and energy within 2^+-60, internal at least 2^-30 of total energy, no
+// component of momentum and field and no psi between 0 and 2^-180, mu0 within 2^+-40.  The smallest numerator is
+// the HLLD's B_n (S_M - v_n): S_M, a quotient of sums that may cancel, is at least 2^-496, B_n 2^-234 and their
+// product with another cancellation 2^-783; the smallest quotient, of it by a denominator up to 2^184, is 2^-967.
+__device__ __forceinline__ bool m_regular64(const double* u, double h) {   // h = 1/(2 mu0)
+    const double re = u[0] * u[4];
+    const double b2 = fma(u[5], u[5], fma(u[6], u[6], fma(u[7], u[7], u[8] * u[8])));
+    const double k2 = fma(u[1], u[1], fma(u[2], u[2], u[3] * u[3]));
+    const double ri = fma(-0.5, k2, u[0] * fma(-h, b2, u[4]));
+    bool ok = within64(u[0], 60) && within64(u[4], 60) && ri >= 0x1p-30 * re;
+#pragma unroll
+    for (int v = 1; v < 9; ++v)
+        if (v != 4) ok = ok && !tiny64(u[v], 0x1p-180);
+    return ok;
 }
 
 }  // namespace nemo

@@ -25,6 +25,40 @@ constexpr int MPB = 2;          // mortars per 128-thread task
 constexpr int scratch_doubles(int V) { return MPB * (V * NF + V * 64 + 4 * V * NF) + 4 * NN * NN; }
 constexpr int SCRATCH_DOUBLES = scratch_doubles(9);
 
+// The surface fluxes in Plain64, out of line: few nodes take them.  States go by value, so that those of the
+// other path stay in registers.
+template <int N>
+struct Vec64 {
+    double v[N];
+};
+
+template <int N>
+__device__ __forceinline__ Vec64<N> vec64(const double* u) {
+    Vec64<N> r;
+#pragma unroll
+    for (int v = 0; v < N; ++v) r.v[v] = u[v];
+    return r;
+}
+
+template <int N>
+__device__ __forceinline__ void take(double* F, const Vec64<N>& r) {
+#pragma unroll
+    for (int v = 0; v < N; ++v) F[v] = r.v[v];
+}
+
+static __device__ __noinline__ Vec64<5> riem64_plain(int kind, Vec64<5> uL, Vec64<5> uR, const OpConsts& k) {
+    Vec64<5> F;
+    riem64<Plain64, false>(kind, uL.v, uR.v, F.v, k);
+    return F;
+}
+
+static __device__ __noinline__ Vec64<9> m_riem64_plain(int kind, Vec64<9> uL, Vec64<9> uR, const OpConsts& k, double ch) {
+    Vec64<9> F;
+    if (kind == NEMO_SURFFLUX_HLLD) m_hlld64<Plain64>(uL.v, uR.v, F.v, mhd64<true>(k, ch));
+    else m_rusanov64<Plain64>(uL.v, uR.v, F.v, mhd64<false>(k, ch));
+    return F;
+}
+
 // LGL-weighted mean of a coarse face trace held as [V][NF] (out of line: taken only on a shock)
 static __device__ __noinline__ void face_mean(const double* uc, int V, double* out, const OpConsts& k) {
     for (int v = 0; v < V; ++v) {
@@ -123,10 +157,12 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
         }
         double F[V], Gf[V], Gc[V];
         double* out = a.mflux + ((5 * m + 1 + kq) * V) * NF + (i + NN * j);
-        if (MHD) {
+        if constexpr (MHD) {
             const double ch = a.ctrl->glm_ch;
-            if (a.surface_flux == NEMO_SURFFLUX_HLLD) m_hlld64(uL, uR, F, mhd64<true>(k, ch));
-            else m_rusanov64(uL, uR, F, mhd64<false>(k, ch));
+            const double h = 0.5 / k.mu0;
+            if (!(k.quick && m_regular64(up, h) && m_regular64(uf, h))) take(F, m_riem64_plain(a.surface_flux, vec64<9>(uL), vec64<9>(uR), k, ch));
+            else if (a.surface_flux == NEMO_SURFFLUX_HLLD) m_hlld64<Quick64>(uL, uR, F, mhd64<true>(k, ch));
+            else m_rusanov64<Quick64>(uL, uR, F, mhd64<false>(k, ch));
             m_nc_x<double>(rf, uL, uR, Gf, k.mu0);
             m_nc_x<double>(rp, uL, uR, Gc, k.mu0);
 #pragma unroll
@@ -135,7 +171,8 @@ __device__ __forceinline__ void mortar_pair(const MortarArgs& a, int64_t pair, d
                 s_fs[ml][kq][v][i + NN * j] = F[v] + Gc[v];
             }
         } else {
-            riemann64(a.surface_flux, uL, uR, F, k);
+            if (!(k.quick && regular64(up) && regular64(uf))) take(F, riem64_plain(a.surface_flux, vec64<5>(uL), vec64<5>(uR), k));
+            else riem64<Quick64, false>(a.surface_flux, uL, uR, F, k);
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 out[v * NF] = F[v];

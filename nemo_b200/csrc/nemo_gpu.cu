@@ -695,6 +695,7 @@ int nemo_gpu_init(const nemo_cfg* cfg) {
     o.repair_decr = cfg->repair_decr;
     o.mu0 = cfg->mu0;
     o.skm1 = 1.0 / o.km1;
+    o.quick = o.km1 >= 0x1p-10 && o.km1 <= 0x1p10 && (!is_mhd() || (o.mu0 >= 0x1p-40 && o.mu0 <= 0x1p40));
     o.cool = cfg->source == NEMO_SOURCE_BAROTROPIC_COOLING ? 1 : 0;
     o.cool_rho = cfg->dens_critical;
     o.cool_ci = cfg->k_isothermal / (cfg->kappa - 1.0);

@@ -4,12 +4,13 @@
 // reference spreads over hook_pre_rk_timestep_300 and hook_mid_rk_timestep_500:
 //   1. the element's state into shared memory, the 96 neighbour trace nodes (or 2:1 mortar flux rows)
 //      beside it by cp.async, in flight while
-//   2. the per-node primitives (velocities, beta_d = rho/(2 p_d) per direction) are computed;
+//   2. the per-node primitives (velocities, beta_d = rho/(2 p_d) per direction) are computed, and the node and
+//      the traces checked for operands that the quotients of ieee64.cuh are not made for;
 //   3. per direction, the 96 two-point fluxes of the split form (16 lines x 6 node pairs), the 32 face
 //      fluxes (kernel_fill_faceflux, source/kernel/mcfv/3d/kernel_flux_mod.f90:47-278) and, where
 //      alpha > 0, the 48 FV subcell fluxes, each an independent task of one thread with its result in
 //      shared memory; then each node sums its own pairs in a fixed order, the surface lift, the FV
-//      term and the convex blend;
+//      term and the convex blend (an element whose check failed does 2 and 3 again with / and sqrt);
 //   4. the LSRK 5-4 register/state update (timedisc_probe, source/timedisc/rungekutta/
 //      low-storage/4-5/timedisc_probe_mod.f90:7-39; rkstep_cb :19-49);
 //   5. the positivity repair (dgfv_repair_3d, source/kernel/mcfv/3d/kernel_validate_mod.f90:159-272);
@@ -277,18 +278,192 @@ __device__ __forceinline__ void epilogue64(const StageArgs& a, double rho, doubl
     }
 }
 
+// Per-node primitives of state q at sp[variable * NP]: velocities and, per direction d, beta_d = rho/(2 p_d),
+// where p_d is the pressure of the state rotated into direction d (the reference evaluates the two-point flux on
+// the rotated state, so the kinetic-energy sum runs in the rotated component order)
+template <class A>
+__device__ __forceinline__ void velocities64(const double* q, const Rcp64& r, double* sp) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sp[c * NP] = A::quot(q[1 + c], r);
+}
+
+template <class A>
+__device__ __forceinline__ void beta64(const double* q, const Rcp64& r, int d, double* sp, const OpConsts& k) {
+#pragma unroll
+    for (int dd = 0; dd < 3; ++dd) {   // q indexed at compile time
+        if (dd != d) continue;
+        const double u[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
+        sp[(3 + dd) * NP] = A::div(0.5 * q[0], pressure64<A>(u, r, k));
+    }
+}
+
+template <class A>
+__device__ __forceinline__ void primitives64(const double* q, const Rcp64& r, double* sp, const OpConsts& k) {
+    velocities64<A>(q, r, sp);
+#pragma unroll
+    for (int dd = 0; dd < 3; ++dd) beta64<A>(q, r, dd, sp, k);
+}
+
+// The fluxes of the 16 lines of direction d into shared memory, by the direction's two warps: two-point fluxes to
+// sF, subcell fluxes to sV, face fluxes in the places of their traces in tr.
+template <class A, bool BLEND, bool FAST>
+__device__ __forceinline__ void fluxes64(int volume_flux, int surface_flux, int d, int w, int lane, double al,
+                                         const double* su, double* tr, double* sF, double* sV, const int32_t* s_nbr,
+                                         const OpConsts& k) {
+    const double* sp = su + (O_SP - O_SU);
+    const int c0 = d, c1 = d == 2 ? 0 : d + 1, c2 = d == 0 ? 2 : d - 1;
+    const double *m0 = su + (1 + c0) * NP, *m1 = su + (1 + c1) * NP, *m2 = su + (1 + c2) * NP;   // momenta
+    constexpr int VEL = O_SP - NP, BETA = O_SP + 2 * NP;   // from a momentum to its velocity, to its beta
+    // ---- two-point fluxes, two pairs of the 16 lines at a time: warp 0 pairs 0, 1, 4, 5, warp 1 pairs 2, 3
+    //      and then the faces (all pairs on warp 0: 396 against 383 us per stage at Sedov 32^3)
+#pragma unroll 1
+    for (int g = w; g < 3; g += 2) {
+        const int pq = 2 * g + (lane >> 4), ab = lane & 15;
+        const int i = line_phys(d, ab, (0x211000 >> (4 * pq)) & 3), m = line_phys(d, ab, (0x332321 >> (4 * pq)) & 3);
+        double F[V];
+        if (!FAST && volume_flux == NEMO_VOLFLUX_CENTRAL) {
+            const double ui[V] = {su[i], m0[i], m1[i], m2[i], su[4 * NP + i]};
+            const double um[V] = {su[m], m0[m], m1[m], m2[m], su[4 * NP + m]};
+            central64<A>(ui, um, F, k);
+        } else {
+            const Node5 ni = {su[i], sp[6 * NP + i], m0[VEL + i], m1[VEL + i], m2[VEL + i], m0[BETA + i]};
+            const Node5 nm = {su[m], sp[6 * NP + m], m0[VEL + m], m1[VEL + m], m2[VEL + m], m0[BETA + m]};
+            chandrashekar64<A>(ni, nm, F, k);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) sF[(v * NPAIR + pq) * FROW + ab] = F[v];
+    }
+    // ---- Riemann fluxes: round 0 the two faces of the 16 lines (warp 1), rounds 1 and 2 the FV subcell
+    //      interfaces 0, 1 (warp 0) and 2 (half of warp 1)
+    const int rounds = BLEND && al > 0.0 ? 3 : 1;
+#pragma unroll 1
+    for (int rt = 1 - w; rt < rounds; rt += 2) {
+        const int hi = lane >> 4, ab = lane & 15;
+        if (rt == 2 && hi) break;
+        const double *pL, *pR;
+        int stL = NP, stR = NP;
+        int32_t ne = 0;
+        double* own_tr = tr + (2 * d + hi) * NF + ab;
+        if (rt == 0) {
+            ne = s_nbr[2 * d + hi];
+            const double* own = su + line_phys(d, ab, hi ? NN - 1 : 0);
+            const double* oth = ne == -1 ? own : own_tr;   // domain boundary: the own trace
+            const int sto = ne == -1 ? NP : 6 * NF;
+            pL = hi ? own : oth;
+            pR = hi ? oth : own;
+            stL = hi ? NP : sto;
+            stR = hi ? sto : NP;
+        } else {
+            const int qi = 2 * (rt - 1) + hi;
+            pL = su + line_phys(d, ab, qi);
+            pR = su + line_phys(d, ab, qi + 1);
+        }
+        const double uL[V] = {pL[0], pL[(1 + c0) * stL], pL[(1 + c1) * stL], pL[(1 + c2) * stL], pL[4 * stL]};
+        const double uR[V] = {pR[0], pR[(1 + c0) * stR], pR[(1 + c1) * stR], pR[(1 + c2) * stR], pR[4 * stR]};
+        double F[V];
+        riem64<A, FAST>(surface_flux, uL, uR, F, k);
+        if (rt == 0) {
+            if (ne > -2) {   // a mortar's flux row is there already
+#pragma unroll
+                for (int v = 0; v < V; ++v) own_tr[v * 6 * NF] = F[v];
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) sV[(v * (NN - 1) + 2 * (rt - 1) + hi) * FROW + ab] = F[v];
+        }
+    }
+}
+
+// Node n's terms of direction d, in that direction's component order
+template <bool BLEND>
+__device__ __forceinline__ void terms64(int d, int n, double al, const double* tr, const double* sF, const double* sV,
+                                        const double* s_S, const double* s_winv, double* t) {
+    // ---- the node's terms: its three pairs in ascending order of the other node, lift, FV, blend
+    const int pos = (n >> (2 * d)) & 3;
+    const int ab = d == 0 ? n >> 2 : (d == 1 ? (n & 3) | ((n >> 4) << 2) : n & 15);
+    const unsigned rows = (unsigned)(0x0542053104300210ull >> (16 * pos));   // pair rows of this position
+#pragma unroll
+    for (int v = 0; v < V; ++v) t[v] = 0.0;
+#pragma unroll
+    for (int mm = 0; mm < NN - 1; ++mm) {
+        const double s = s_S[pos * NN + mm + (mm >= pos ? 1 : 0)];
+        const double* f = sF + ((rows >> (4 * mm)) & 15) * FROW + ab;
+#pragma unroll
+        for (int v = 0; v < V; ++v) t[v] = t[v] + s * f[v * NPAIR * FROW];
+    }
+    const double wi = s_winv[pos];
+    const double* sS = tr + 2 * d * NF + ab;   // face fluxes of the line: [v][2][NF]
+    if (pos == 0) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) t[v] = t[v] + wi * (-sS[v * 6 * NF]);
+    }
+    if (pos == NN - 1) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) t[v] = t[v] + wi * sS[v * 6 * NF + NF];
+    }
+    if (BLEND && al > 0.0) {
+        const double* fl = pos == 0 ? sS : sV + (pos - 1) * FROW + ab;
+        const double* fr = pos == NN - 1 ? sS + NF : sV + pos * FROW + ab;
+        const int sl = pos == 0 ? 6 * NF : (NN - 1) * FROW, sr = pos == NN - 1 ? 6 * NF : (NN - 1) * FROW;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const double fv = wi * (fr[v * sr] - fl[v * sl]);
+            t[v] = (1.0 - al) * t[v] + al * fv;
+        }
+    }
+}
+
+__device__ __forceinline__ void pair_sync(int bar) { asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory"); }
+
+// The node's rhs terms with the language's own quotients, by 64 threads that meet at barrier bar.  Out of line:
+// for elements that are not regular, or border one that is not.  The face fluxes of the first attempt stand in
+// the places of the traces, so these are fetched again.
+struct Terms64 {
+    double v[V];
+};
+__device__ __noinline__ Terms64 plain_terms64(const StageArgs& a, double al, int bar) {
+    extern __shared__ __align__(16) double smem[];
+    const OpConsts& k = c_ops64;
+    const int64_t e = a.E_begin + blockIdx.x;
+    const int n = threadIdx.x, lane = n & 31, w = n >> 5, pn = phys(n);
+    double *su = smem + O_SU, *sp = smem + O_SP, *tr = smem + O_TR, *sF = smem + O_SF, *sV = smem + O_SV;
+    pair_sync(bar);
+    double q[V];
+    for (int v = 0; v < V; ++v) q[v] = su[v * NP + pn];
+    primitives64<Plain64>(q, Plain64::rcp(q[0]), sp + pn, k);
+    for (int p = n; p < 6 * NF; p += TPE) {
+        const int f = p >> 4, ab = p & 15, ne = a.nbr[e * 6 + f];
+        if (ne < 0) continue;   // a mortar's flux row is as it was
+        const int m = line_node(f >> 1, ab & 3, ab >> 2, (f & 1) ? 0 : NN - 1);
+        for (int v = 0; v < V; ++v) tr[v * 6 * NF + p] = a.u_in[((int64_t)v * a.E + ne) * NP + m];
+    }
+    pair_sync(bar);
+    Terms64 R;
+    for (int d = 0; d < 3; ++d) {
+        fluxes64<Plain64, true, false>(a.volume_flux, a.surface_flux, d, w, lane, al, su, tr, sF, sV, a.nbr + e * 6, k);
+        pair_sync(bar);
+        double t[V];
+        terms64<true>(d, n, al, tr, sF, sV, k.S, k.winv, t);
+        pair_sync(bar);
+        const double cd = a.cdel[e * 3 + d];
+        const int o[V] = {0, 1 + d, 1 + (d + 1) % 3, 1 + (d + 2) % 3, 4};
+        for (int v = 0; v < V; ++v) R.v[o[v]] = d == 0 ? cd * t[v] : R.v[o[v]] + cd * t[v];
+    }
+    return R;
+}
+
 }  // namespace
 
 // ND directions at a time, each by a group of 64 threads with its own flux arrays.  ND = 1 (64 threads) packs
 // an SM with elements; ND = 3 (192 threads) runs an element's directions side by side, which shortens the
 // element (26 k cycles alone, 18 k of them the directions) when there are too few to fill the SMs anyway.
 template <int ND, bool BLEND, bool RHS_ONLY, bool FAST>
-__global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageArgs a) {
+__global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(const __grid_constant__ StageArgs a) {
     extern __shared__ __align__(16) double smem[];
     __shared__ double s_S[NN * NN], s_winv[NN], s_vi[NN * NN];   // operator rows, indexed per thread
     __shared__ double s_alpha;
     __shared__ unsigned long long s_lam[2][4];
-    __shared__ int s_bad;
+    __shared__ int s_bad, s_plain;
     __shared__ int32_t s_nbr[6];
 
     const OpConsts& k = c_ops64;
@@ -308,7 +483,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
     for (int r = 0; r < FETCH; ++r)
         nes[r] = (ND == 1 && r == 0) || tid + r * TPE < 6 * NF ? __ldg(a.nbr + e * 6 + 4 * r + (tid >> 4)) : -1;
     dep_sync();
-    if (!RHS_ONLY && ctrl->done && !a.prep_only) return;
+    const int32_t done = RHS_ONLY ? 0 : ctrl->done;   // looked at when the loads below are under way
     double* const su = smem + O_SU;
     double* const sp = smem + O_SP;
     double* const tr = smem + O_TR;
@@ -320,6 +495,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
     double q[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) q[v] = __ldcg(a.u_in + ((int64_t)v * E + e) * NP + n);
+    if (done && !a.prep_only) return;
     auto epilogue = [&]() {
         epilogue64<ND>(a, q[0], pressure64(q, k), sp, s_vi, s_lam, e, n, k, [&](int dd) {
             const double rr[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
@@ -351,29 +527,36 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
     }
     if (!RHS_ONLY && a.stage > 0 && tid < 4 * V)   // the register rows (four lines each), needed at the end
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.reg + ((int64_t)(tid >> 2) * E + e) * NP + 16 * (tid & 3)));
-    if (tid == 0) s_bad = 0;
+    if (tid == 0) s_bad = s_plain = 0;
     if (BLEND && tid < 32) smooth_alpha64(a, e, lane, &s_alpha);
 
-    // per-node primitives: velocities and, per direction d, beta_d = rho/(2 p_d) where p_d is the
-    // pressure of the state rotated into direction d (the reference evaluates the two-point flux on
-    // the rotated state, so the kinetic-energy sum runs in the rotated component order)
     const int pn = phys(n);
     const Rcp64 ir = rcp64r(q[0]);
     if (dg == 0) {
 #pragma unroll
         for (int v = 0; v < V; ++v) su[v * NP + pn] = q[v];
         sp[6 * NP + pn] = ir.y;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sp[c * NP + pn] = quot64(q[1 + c], ir);
     }
-#pragma unroll
-    for (int dd = 0; dd < 3; ++dd) {
-        if (ND == 3 && dd != dg) continue;
-        const double r[V] = {q[0], q[1 + dd], q[1 + (dd + 1) % 3], q[1 + (dd + 2) % 3], q[4]};
-        sp[(3 + dd) * NP + pn] = div64(0.5 * q[0], pressure64(r, ir, k));
+    if (ND == 1) {
+        primitives64<Quick64>(q, ir, sp + pn, k);
+    } else {
+        if (dg == 0) velocities64<Quick64>(q, ir, sp + pn);
+        beta64<Quick64>(q, ir, dg, sp + pn, k);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    // Whether this node and the traces this thread fetched keep to the domain of Quick64.  Looked at after the first
+    // direction (a vote here, or the second attempt inside the loop, costs more).  us per stage without -> with it:
+    // Sedov 32^3 379 -> 392, the 24k-element forest 333 -> 350, smooth 16^3 44.8 -> 46.1, 4^3 9.4 -> 9.4.
+    bool regular = k.quick && regular64(q);
+#pragma unroll
+    for (int r = 0; r < FETCH; ++r) {
+        if (nes[r] < 0) continue;
+        const double* o = tr + tid + r * TPE;
+        const double uo[V] = {o[0], o[6 * NF], o[2 * 6 * NF], o[3 * 6 * NF], o[4 * 6 * NF]};
+        regular = regular && regular64(uo);
+    }
     __syncthreads();
+    if (!regular) s_plain = 1;
     const double al = BLEND ? s_alpha : 0.0;
 
     // The node's rhs terms, in the component order of the current direction: after each direction the
@@ -384,101 +567,10 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
 #pragma unroll 1
     for (int d = dg; d < (ND == 1 ? 3 : dg + 1); ++d) {
         const int c0 = d, c1 = d == 2 ? 0 : d + 1, c2 = d == 0 ? 2 : d - 1;
-        const double *m0 = su + (1 + c0) * NP, *m1 = su + (1 + c1) * NP, *m2 = su + (1 + c2) * NP;   // momenta
-        constexpr int VEL = O_SP - NP, BETA = O_SP + 2 * NP;   // from a momentum to its velocity, to its beta
-        // ---- two-point fluxes, two pairs of the 16 lines at a time: warp 0 pairs 0, 1, 4, 5, warp 1 pairs 2, 3
-        //      and then the faces (all pairs on warp 0: 396 against 383 us per stage at Sedov 32^3)
-#pragma unroll 1
-        for (int g = w; g < 3; g += 2) {
-            const int pq = 2 * g + (lane >> 4), ab = lane & 15;
-            const int i = line_phys(d, ab, (0x211000 >> (4 * pq)) & 3), m = line_phys(d, ab, (0x332321 >> (4 * pq)) & 3);
-            double F[V];
-            if (!FAST && a.volume_flux == NEMO_VOLFLUX_CENTRAL) {
-                const double ui[V] = {su[i], m0[i], m1[i], m2[i], su[4 * NP + i]};
-                const double um[V] = {su[m], m0[m], m1[m], m2[m], su[4 * NP + m]};
-                central64(ui, um, F, k);
-            } else {
-                const Node5 ni = {su[i], sp[6 * NP + i], m0[VEL + i], m1[VEL + i], m2[VEL + i], m0[BETA + i]};
-                const Node5 nm = {su[m], sp[6 * NP + m], m0[VEL + m], m1[VEL + m], m2[VEL + m], m0[BETA + m]};
-                chandrashekar64(ni, nm, F, k);
-            }
-#pragma unroll
-            for (int v = 0; v < V; ++v) sF[(v * NPAIR + pq) * FROW + ab] = F[v];
-        }
-        // ---- Riemann fluxes: round 0 the two faces of the 16 lines (warp 1), rounds 1 and 2 the FV subcell
-        //      interfaces 0, 1 (warp 0) and 2 (half of warp 1)
-        const int rounds = BLEND && al > 0.0 ? 3 : 1;
-#pragma unroll 1
-        for (int rt = 1 - w; rt < rounds; rt += 2) {
-            const int hi = lane >> 4, ab = lane & 15;
-            if (rt == 2 && hi) break;
-            const double *pL, *pR;
-            int stL = NP, stR = NP;
-            int32_t ne = 0;
-            double* own_tr = tr + (2 * d + hi) * NF + ab;
-            if (rt == 0) {
-                ne = s_nbr[2 * d + hi];
-                const double* own = su + line_phys(d, ab, hi ? NN - 1 : 0);
-                const double* oth = ne == -1 ? own : own_tr;   // domain boundary: the own trace
-                const int sto = ne == -1 ? NP : 6 * NF;
-                pL = hi ? own : oth;
-                pR = hi ? oth : own;
-                stL = hi ? NP : sto;
-                stR = hi ? sto : NP;
-            } else {
-                const int qi = 2 * (rt - 1) + hi;
-                pL = su + line_phys(d, ab, qi);
-                pR = su + line_phys(d, ab, qi + 1);
-            }
-            const double uL[V] = {pL[0], pL[(1 + c0) * stL], pL[(1 + c1) * stL], pL[(1 + c2) * stL], pL[4 * stL]};
-            const double uR[V] = {pR[0], pR[(1 + c0) * stR], pR[(1 + c1) * stR], pR[(1 + c2) * stR], pR[4 * stR]};
-            double F[V];
-            riem64<FAST>(a.surface_flux, uL, uR, F, k);
-            if (rt == 0) {
-                if (ne > -2) {   // a mortar's flux row is there already
-#pragma unroll
-                    for (int v = 0; v < V; ++v) own_tr[v * 6 * NF] = F[v];
-                }
-            } else {
-#pragma unroll
-                for (int v = 0; v < V; ++v) sV[(v * (NN - 1) + 2 * (rt - 1) + hi) * FROW + ab] = F[v];
-            }
-        }
+        fluxes64<Quick64, BLEND, FAST>(a.volume_flux, a.surface_flux, d, w, lane, al, su, tr, sF, sV, s_nbr, k);
         group_sync<ND>(dg);
-        // ---- the node's terms: its three pairs in ascending order of the other node, lift, FV, blend
-        const int pos = (n >> (2 * d)) & 3;
-        const int ab = d == 0 ? n >> 2 : (d == 1 ? (n & 3) | ((n >> 4) << 2) : n & 15);
-        const unsigned rows = (unsigned)(0x0542053104300210ull >> (16 * pos));   // pair rows of this position
         double t[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) t[v] = 0.0;
-#pragma unroll
-        for (int mm = 0; mm < NN - 1; ++mm) {
-            const double s = s_S[pos * NN + mm + (mm >= pos ? 1 : 0)];
-            const double* f = sF + ((rows >> (4 * mm)) & 15) * FROW + ab;
-#pragma unroll
-            for (int v = 0; v < V; ++v) t[v] = t[v] + s * f[v * NPAIR * FROW];
-        }
-        const double wi = s_winv[pos];
-        const double* sS = tr + 2 * d * NF + ab;   // face fluxes of the line: [v][2][NF]
-        if (pos == 0) {
-#pragma unroll
-            for (int v = 0; v < V; ++v) t[v] = t[v] + wi * (-sS[v * 6 * NF]);
-        }
-        if (pos == NN - 1) {
-#pragma unroll
-            for (int v = 0; v < V; ++v) t[v] = t[v] + wi * sS[v * 6 * NF + NF];
-        }
-        if (BLEND && al > 0.0) {
-            const double* fl = pos == 0 ? sS : sV + (pos - 1) * FROW + ab;
-            const double* fr = pos == NN - 1 ? sS + NF : sV + pos * FROW + ab;
-            const int sl = pos == 0 ? 6 * NF : (NN - 1) * FROW, sr = pos == NN - 1 ? 6 * NF : (NN - 1) * FROW;
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const double fv = wi * (fr[v * sr] - fl[v * sl]);
-                t[v] = (1.0 - al) * t[v] + al * fv;
-            }
-        }
+        terms64<BLEND>(d, n, al, tr, sF, sV, s_S, s_winv, t);
         const double cd = __ldg(a.cdel + e * 3 + d);
         if (ND == 3) {
 #pragma unroll
@@ -501,6 +593,7 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
             R[3] = r[1];
             R[4] = r[4];
             __syncthreads();
+            if (s_plain) break;
         }
     }
     if (ND == 3) {
@@ -508,6 +601,11 @@ __global__ void __launch_bounds__(ND * TPE, CTAS64 / ND) k_stage_euler64(StageAr
         if (dg != 0) return;   // the rest is group 0's
 #pragma unroll
         for (int v = 0; v < V; ++v) R[v] = (R[v] + sR[v * NP + n]) + sR[(V + v) * NP + n];
+    }
+    if (s_plain) {
+        const Terms64 p = plain_terms64(a, al, ND == 1 ? 0 : 1);
+#pragma unroll
+        for (int v = 0; v < V; ++v) R[v] = p.v[v];
     }
 
     // ---- rhs, LSRK register and state update

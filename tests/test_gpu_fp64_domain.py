@@ -1,0 +1,155 @@
+"""The plain FP64 forms where their own quotients and roots end: ieee64.cuh against / and sqrt bit for bit over the
+stated domain, and states outside it -- momenta and fields down to the smallest denormal, units that make
+densities and pressures huge or minute, densities that differ by hundreds of orders of magnitude, zero pressure,
+velocities far above the sound speed -- alone and beside ordinary elements, in both widths of the Euler kernel, on
+open boundaries and on 2:1 faces.  Everything equals the oracle bit for bit, NaN where it has NaN: the plain path's
+contract leaves no tolerance."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from nemo_b200 import abi, mesh, setups
+from nemo_b200 import build as nb
+from nemo_b200.solver import Solver
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(autouse=True)
+def _fin():
+    yield
+    try:
+        abi.call("nemo_gpu_finalize")
+    except Exception:
+        pass
+
+
+def test_quotients_and_roots(tmp_path):
+    lib = str(tmp_path / "quotients_check.so")
+    subprocess.run([nb.nvcc(), *nb.ARCH, "-O3", "-std=c++17", "-fmad=false", "-shared", "-Xcompiler", "-fPIC",
+                    os.path.join(HERE, "quotients_check.cu"), "-o", lib], check=True)
+    bad = (ctypes.c_ulonglong * 7)()
+    assert ctypes.CDLL(lib).quotients_check(200, 1000, bad) == 0
+    assert bad[6] > 10 ** 8          # 151 552 threads x 200 rounds, a few near ties in each
+    assert list(bad)[:6] == [0] * 6
+
+
+MESHES = {
+    "4^3": lambda: mesh.brick(4),
+    "13x13x11": lambda: mesh.brick(13, 13, 11),      # one direction at a time (above 12 elements per SM)
+    "open": lambda: mesh.brick(5, 3, 2, periodic=(False,) * 3),
+    "forest": lambda: mesh.forest(2, lambda lvl, c, s: c[:, 1] < 0.5, max_level=1),
+}
+
+
+def spread(rng, shape, lo, hi):
+    """Random numbers with exponents from lo to hi, a third of them zeros of either sign."""
+    x = np.ldexp(rng.uniform(1, 2, shape) * rng.choice([-1.0, 1.0], shape), rng.integers(lo, hi, shape))
+    return np.where(rng.random(shape) < 1 / 3, rng.choice([0.0, -0.0], shape), x)
+
+
+def ordinary(m, mhd):
+    u = setups.smooth_random(m, seed=5, kappa=5.0 / 3.0 if mhd else 1.4)
+    if mhd:
+        x, y, z = m.node_coords(setups.LGL4)
+        b = [0.3 + 0.2 * np.sin(2 * np.pi * (x + y)), -0.1 * np.cos(2 * np.pi * z), 0.15 * np.sin(2 * np.pi * (y - z)),
+             0.02 * np.cos(2 * np.pi * x)]
+        u = np.concatenate([u, np.stack(b)])
+        u[4] += 0.5 * sum(v ** 2 for v in b)
+    u[:5, :, 17] *= 1.5     # jumps between some nodes: alpha > 0 in part of the elements
+    u[4, :, 17] += 1.0
+    return u
+
+
+def still(u, rng, lo, hi):
+    """At rest but for momenta (and a field) of exponents lo..hi, in every other element."""
+    e = slice(0, None, 2)
+    u[4, e] -= 0.5 * (u[1:4, e] ** 2).sum(0) / u[0, e]
+    u[1:4, e] = spread(rng, u[1:4, e].shape, lo, hi)
+    if len(u) == 9:
+        u[4, e] -= 0.5 * (u[5:, e] ** 2).sum(0)
+        u[5:, e] = spread(rng, u[5:, e].shape, lo, hi)
+
+
+def scaled(u, k):
+    """In units in which densities and energies are 2^k times as large."""
+    u[:5] *= 2.0 ** k
+    u[5:] *= 2.0 ** (k // 2)
+
+
+def fast(u, rng):
+    k = rng.random(u.shape[1:]) < 0.3
+    u[1][k] = 1e12 * rng.choice([-1.0, 1.0], k.sum())
+    u[4][k] = 0.5 * u[1][k] ** 2 / u[0][k] * (1 + 1e-13) + 2
+
+
+def empty(u, rng):
+    k = rng.random(u.shape[1:]) < 0.02
+    u[1:, k] = 0.0
+
+
+STATES = {
+    "denormal momenta": lambda u, rng: still(u, rng, -1074, -900),
+    "minute momenta": lambda u, rng: still(u, rng, -560, -20),
+    "huge units": lambda u, rng: scaled(u, 200),
+    "minute units": lambda u, rng: scaled(u, -990),
+    "edge of the regular range": lambda u, rng: scaled(u, -100 if len(u) == 5 else -60),
+    "mixed densities": lambda u, rng: np.multiply(u[:5], 2.0 ** rng.integers(-300, 300, u.shape[1:]), out=u[:5]),
+    "zero pressure": empty,
+    "velocity far above sound": fast,
+}
+
+
+@pytest.mark.parametrize("faces", ["default", "rusanov"])
+@pytest.mark.parametrize("mhd", [False, True])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_states_outside_the_domain(name, mhd, faces):
+    m = MESHES[name]()
+    kw = dict(positivity=0)
+    if mhd:
+        kw.update(eqn=abi.EQN_MHD, n_vars=9, kappa=5.0 / 3.0, volume_flux=abi.VOLFLUX_EC_MHD, surface_flux=abi.SURFFLUX_HLLD,
+                  glm_ch=0.7, glm_alpha=0.3)
+    if faces == "rusanov":
+        kw.update(surface_flux=abi.SURFFLUX_RUSANOV, volume_flux=abi.VOLFLUX_CENTRAL)
+    for ind in (abi.IND_NONE, abi.IND_MODAL):
+        c = abi.default_cfg(indicator=ind, **kw)
+        s = Solver(c, m)
+        o = orc.Oracle.for_mesh(c, m)
+        for label, make in STATES.items():
+            u = ordinary(m, mhd)
+            make(u, np.random.default_rng(7))
+            u = np.ascontiguousarray(u)
+            s.upload(u)
+            ref = o.rhs(u, alpha=o.alpha(u)) if ind == abi.IND_MODAL else o.rhs(u)
+            assert np.array_equal(s.rhs(), ref, equal_nan=True), (label, ind)
+        s.finalize()
+
+
+@pytest.mark.parametrize("kappa", [1.0 + 2.0 ** -30, 5000.0])
+def test_extreme_kappa(kappa):
+    """Outside the range of kappa for which the flux quotients stay in their domain."""
+    m = MESHES["4^3"]()
+    c = abi.default_cfg(indicator=abi.IND_MODAL, kappa=kappa)
+    u = np.ascontiguousarray(ordinary(m, False))
+    s = Solver(c, m)
+    s.upload(u)
+    o = orc.Oracle.for_mesh(c, m)
+    assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)), equal_nan=True)
+
+
+def test_steps_through_a_still_ambient():
+    """A blast in a still ambient, whose momenta fall off through hundreds of orders of magnitude ahead of it: 40 steps
+    on 20^3 elements in the oracle's bits."""
+    m = mesh.brick(20, lo=(-0.5,) * 3, hi=(0.5,) * 3)
+    u = setups.sedov(m, sigma=0.05)
+    c = abi.default_cfg(indicator=abi.IND_MODAL, positivity=1, cfl=0.5)
+    s = Solver(c, m)
+    s.upload(u)
+    t, n = s.run(nsteps=40)
+    ref, tr, nr, _ = orc.Oracle.for_mesh(c, m).run(u, nsteps=40)
+    assert t == tr and n == nr and np.array_equal(s.download(), ref)
