@@ -1,27 +1,16 @@
 // mhd_phys.cuh -- GLM-MHD physics for the stage kernels, templated on the arithmetic type.
 //
-// R = double (plain path, compiled with -fmad=false): the reference's expressions in the
-// reference's order, bit-identical to oracle/nemo_oracle.cpp.  R = float (FP32 form, fast math):
-// the same formulas in FP32, with the logarithmic-mean switch widened to f^2 < 1e-2.
+// R = float: the FP32 form's fluxes (fast math), with the logarithmic-mean switch widened to f^2 < 1e-2.
+// R = double: pressure, admissibility, wave speed and non-conservative term wherever they are taken in FP64, the
+// reference's expressions in the reference's order (-fmad=false where the plain path takes them); the fluxes of the
+// plain path are in mhd_fp64.cuh.
 // All functions work in the frame rotated into the face normal: u = (rho, m_n, m_t1, m_t2, E,
 // B_n, B_t1, B_t2, psi) (source/equations/mhd/equations_mod.f90:141-219).
 #pragma once
 
 #include "common.cuh"
-#include "pmath64.cuh"
 
 namespace nemo {
-
-struct MhdK {
-    double kappa, mu0;
-};
-
-template <typename R>
-__device__ __forceinline__ R mlog(R x);
-template <>
-__device__ __forceinline__ double mlog<double>(double x) { return plog64(x); }
-template <>
-__device__ __forceinline__ float mlog<float>(float x) { return __logf(x); }
 
 // pressure_elemental, source/equations/mhd/equations_mod.f90:223-234
 template <typename R>
@@ -256,9 +245,8 @@ template <typename R>
 __device__ __forceinline__ R ln_mean_rel(R aL, R aR) {
     const R Xi = aR / aL;
     const R u = (Xi * (Xi - R(2.0)) + R(1.0)) / (Xi * (Xi + R(2.0)) + R(1.0));
-    const R eps = sizeof(R) == 8 ? R(1.0e-4) : R(1.0e-2);
-    if (u < eps) return (aL + aR) * R(52.5) / (R(105.0) + u * (R(35.0) + u * (R(21.0) + u * R(15.0))));
-    return (aR - aL) / mlog(Xi);
+    if (u < R(1.0e-2)) return (aL + aR) * R(52.5) / (R(105.0) + u * (R(35.0) + u * (R(21.0) + u * R(15.0))));
+    return (aR - aL) / __logf(Xi);
 }
 
 // EC (Derigs) flux, source/equations/mhd/two_point/ec/two_point_flux_mod.f90:13-86

@@ -133,13 +133,10 @@ __device__ __forceinline__ float hmin16m(float v) {
     return v;
 }
 
-__device__ __forceinline__ double silu_m(double x) { return x / (1.0 + pexp64(-x)); }
 __device__ __forceinline__ float silu_m(float x) { return x / (1.0f + __expf(-x)); }
-__device__ __forceinline__ double expneg(double x) { return pexp64(x); }
-__device__ __forceinline__ float expneg(float x) { return __expf(x); }
 
-// Epilogue: modal (or learned) blending coefficient of the state in su and the CFL bound; sums in
-// the oracle's serial order (one thread per element), MLP layers over 32 threads per element.
+// Epilogue: modal (or learned) blending coefficient of the state in su, its sums shared by the element's 16 threads
+// and the MLP layers over 32 threads per element, and the CFL bound in FP64.
 template <typename R>
 __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsigned long long (*s_lam)[3],
                              unsigned long long* s_vmax, int nel, int64_t e0, int tid, const OpConsts& k) {
@@ -170,7 +167,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
                 const int ai = n % NN, j = (n / NN) % NN, kk = n / NF;
                 R s = R(0.0);
 #pragma unroll
-                for (int i = 0; i < NN; ++i) s = s + op_Vinv<R>(k, ai * NN + i) * q[pel * NP + nidx(i, j, kk)];
+                for (int i = 0; i < NN; ++i) s = s + k.Vinv32[ai * NN + i] * q[pel * NP + nidx(i, j, kk)];
                 t1[pel * NP + n] = s;
             }
             __syncthreads();
@@ -179,7 +176,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
                 const int ai = n % NN, bj = (n / NN) % NN, kk = n / NF;
                 R s = R(0.0);
 #pragma unroll
-                for (int j = 0; j < NN; ++j) s = s + op_Vinv<R>(k, bj * NN + j) * t1[pel * NP + nidx(ai, j, kk)];
+                for (int j = 0; j < NN; ++j) s = s + k.Vinv32[bj * NN + j] * t1[pel * NP + nidx(ai, j, kk)];
                 t2[pel * NP + n] = s;
             }
             __syncthreads();
@@ -188,7 +185,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
                 const int ai = n % NN, bj = (n / NN) % NN, cc = n / NF;
                 R s = R(0.0);
 #pragma unroll
-                for (int kk = 0; kk < NN; ++kk) s = s + op_Vinv<R>(k, cc * NN + kk) * t2[pel * NP + nidx(ai, bj, kk)];
+                for (int kk = 0; kk < NN; ++kk) s = s + k.Vinv32[cc * NN + kk] * t2[pel * NP + nidx(ai, bj, kk)];
                 cm[pel * NP + n] = s;
             }
             __syncthreads();
@@ -302,7 +299,7 @@ __device__ void epilogue_mhd(const StageArgs& a, const double* su, R* scr, unsig
             if (tid < nel) {
                 R z = W3[32];
                 for (int j = 0; j < 32; ++j) z = z + W3[j] * h2[tid * 32 + j];
-                R al = (R)k.alpha_max / (R(1.0) + expneg(-z));
+                R al = (R)k.alpha_max / (R(1.0) + __expf(-z));
                 if (al < (R)k.alpha_min) al = R(0.0);
                 const R am = s_am[tid];
                 if (s_fb[tid]) {
@@ -495,7 +492,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
                     else m_ec_x(ui, um, F, kap, mu0, ch);
                     m_nc_x(ui, ui, um, Gi, mu0);
                     m_nc_x(um, ui, um, Gm, mu0);
-                    const R sim = op_S<R>(k, i * NN + m), smi = op_S<R>(k, m * NN + i);
+                    const R sim = k.S32[i * NN + m], smi = k.S32[m * NN + i];
 #pragma unroll
                     for (int v = 0; v < MV; ++v) {
                         t[i][v] = t[i][v] + sim * (F[v] + Gi[v]);
@@ -505,8 +502,8 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
             // ---- lift
 #pragma unroll
             for (int v = 0; v < MV; ++v) {
-                t[0][v] = t[0][v] + op_winv<R>(k, 0) * (-Fs[0][v]);
-                t[NN - 1][v] = t[NN - 1][v] + op_winv<R>(k, NN - 1) * Fs[1][v];
+                t[0][v] = t[0][v] + k.winv32[0] * (-Fs[0][v]);
+                t[NN - 1][v] = t[NN - 1][v] + k.winv32[NN - 1] * Fs[1][v];
             }
             // ---- FV subcells and blend
             if (BLEND) {
@@ -547,7 +544,7 @@ __global__ void __launch_bounds__(mhd::NT, NEMO_MHD32_MINB) k_stage_mhd(StageArg
 #pragma unroll
                             for (int v = 0; v < MV; ++v) FR[v] = Fs[1][v];
                         }
-                        const R wi = op_winv<R>(k, i);
+                        const R wi = k.winv32[i];
 #pragma unroll
                         for (int v = 0; v < MV; ++v) t[i][v] = (R(1.0) - al) * t[i][v] + al * (wi * (FR[v] - FL[v]));
                     }
