@@ -181,15 +181,15 @@ __device__ __forceinline__ void central64(const double* u, const double* v, doub
 // numerator (the product of two momenta in the mean over the fan) is 2^-891 and the smallest quotient 2^-997.
 // Ordinary flows meet the last condition: in a still ambient the exponents of the momenta double with every few
 // elements from the disturbance (2^-229 on Sedov 32^3 after 40 steps).  A NaN fails the comparisons.
-__device__ __forceinline__ bool within64(double x, int e) {   // 2^-e <= x < 2^e
-    return (unsigned)__double2hiint(x) - ((1023u - e) << 20) < (unsigned)(2 * e) << 20;
+__device__ __forceinline__ bool within64(double x, int lo, int hi) {   // 2^lo <= x < 2^hi
+    return (unsigned)__double2hiint(x) - ((unsigned)(1023 + lo) << 20) < (unsigned)(hi - lo) << 20;
 }
 __device__ __forceinline__ bool tiny64(double x, double limit) { return fabs(x) < limit && x != 0.0; }
 
 __device__ __forceinline__ bool regular64(const double* u) {
     const double re = u[0] * u[4];
     const double ri = fma(-0.5, fma(u[1], u[1], fma(u[2], u[2], u[3] * u[3])), re);
-    return within64(u[0], 100) && within64(u[4], 100) && ri >= 0x1p-30 * re && !tiny64(u[1], 0x1p-280) &&
+    return within64(u[0], -100, 100) && within64(u[4], -100, 100) && ri >= 0x1p-30 * re && !tiny64(u[1], 0x1p-280) &&
            !tiny64(u[2], 0x1p-280) && !tiny64(u[3], 0x1p-280);
 }
 

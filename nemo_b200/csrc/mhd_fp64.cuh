@@ -299,19 +299,20 @@ __device__ __forceinline__ void m_add_nc64(double* F, const double* v, const dou
     F[8] = F[8] + gv;
 }
 
-// As regular64 (euler_fp64.cuh): density and energy within 2^+-60, internal at least 2^-30 of total energy, no
-// component of momentum and field and no psi between 0 and 2^-180, mu0 within 2^+-40.  The smallest numerator is
-// the HLLD's B_n (S_M - v_n): S_M, a quotient of sums that may cancel, is at least 2^-496, B_n 2^-234 and their
-// product with another cancellation 2^-783; the smallest quotient, of it by a denominator up to 2^184, is 2^-967.
+// As regular64 (euler_fp64.cuh): density within 2^-100..2^40 and energy within 2^+-60 (code units, SI, and CGS down to
+// 1e-30 g/cm^3), internal at least 2^-30 of total energy, no component of momentum and field and no psi between 0 and
+// 2^-170, mu0 within 2^+-40.  The smallest numerator is the HLLD's B_n (S_M - v_n): S_M, a quotient of sums that may
+// cancel, is at least 2^-493, B_n 2^-224 and their product with another cancellation 2^-770; the smallest quotient,
+// of it by a denominator up to 2^218, is 2^-988.
 __device__ __forceinline__ bool m_regular64(const double* u, double h) {   // h = 1/(2 mu0)
     const double re = u[0] * u[4];
     const double b2 = fma(u[5], u[5], fma(u[6], u[6], fma(u[7], u[7], u[8] * u[8])));
     const double k2 = fma(u[1], u[1], fma(u[2], u[2], u[3] * u[3]));
     const double ri = fma(-0.5, k2, u[0] * fma(-h, b2, u[4]));
-    bool ok = within64(u[0], 60) && within64(u[4], 60) && ri >= 0x1p-30 * re;
+    bool ok = within64(u[0], -100, 40) && within64(u[4], -60, 60) && ri >= 0x1p-30 * re;
 #pragma unroll
     for (int v = 1; v < 9; ++v)
-        if (v != 4) ok = ok && !tiny64(u[v], 0x1p-180);
+        if (v != 4) ok = ok && !tiny64(u[v], 0x1p-170);
     return ok;
 }
 

@@ -733,7 +733,7 @@ __device__ __forceinline__ void tile32(const StageArgs& a, const Smem32& S, int6
                         const double m2 = __ldcg(g + ((int64_t)(1 + c2) * E + ne) * NP + nn);
                         const double en = __ldcg(g + ((int64_t)4 * E + ne) * NP + nn);
                         // 1/r, for an ordinary density without the compiler's branches
-                        const double ir = within64(r, 1000) ? quot64(1.0, rcp64r(r)) : 1.0 / r;
+                        const double ir = within64(r, -1000, 1000) ? quot64(1.0, rcp64r(r)) : 1.0 / r;
                         const double v0 = m0 * ir, v1 = m1 * ir, v2 = m2 * ir;
                         qn.rho = (float)r;
                         qn.vn = (float)v0;

@@ -82,6 +82,14 @@ def scaled(u, k):
     u[5:] *= 2.0 ** (k // 2)
 
 
+def units(u, rho, v):
+    """Densities rho and velocities v times as large."""
+    u[0] *= rho
+    u[1:4] *= rho * v
+    u[4] *= rho * v * v
+    u[5:] *= np.sqrt(rho) * v
+
+
 def fast(u, rng):
     k = rng.random(u.shape[1:]) < 0.3
     u[1][k] = 1e12 * rng.choice([-1.0, 1.0], k.sum())
@@ -99,6 +107,7 @@ STATES = {
     "huge units": lambda u, rng: scaled(u, 200),
     "minute units": lambda u, rng: scaled(u, -990),
     "edge of the regular range": lambda u, rng: scaled(u, -100 if len(u) == 5 else -60),
+    "CGS units of the interstellar medium": lambda u, rng: units(u, 2.0 ** -80, 2.0 ** 20),
     "mixed densities": lambda u, rng: np.multiply(u[:5], 2.0 ** rng.integers(-300, 300, u.shape[1:]), out=u[:5]),
     "zero pressure": empty,
     "velocity far above sound": fast,
