@@ -162,3 +162,46 @@ def test_steps_through_a_still_ambient():
     t, n = s.run(nsteps=40)
     ref, tr, nr, _ = orc.Oracle.for_mesh(c, m).run(u, nsteps=40)
     assert t == tr and n == nr and np.array_equal(s.download(), ref)
+
+
+def corners(rng, shape, mhd):
+    """States all over the regular range and its edges: every node its own density and energy, up to velocities and
+    fields that leave 2^-30 of the energy to the pressure, and components down to the smallest that count."""
+    lo, hi, elo, ehi, tiny = (-100, 40, -60, 60, -170) if mhd else (-100, 100, -100, 100, -280)
+
+    def exponents(a, b):
+        x = rng.uniform(a, b, shape)
+        return np.where(rng.random(shape) < 0.3, rng.choice([a + 0.01, b - 0.01], shape), x)
+
+    rho, en = 2.0 ** exponents(lo, hi), 2.0 ** exponents(elo, ehi)
+    n = 7 if mhd else 3
+    share = rng.dirichlet(np.ones(n), shape) * np.where(rng.random(shape) < 0.5, 1 - 2.0 ** -29, 0.5)[..., None]
+    top = [np.sqrt(2 * share[..., c] * en * (rho if c < 3 else 1.0)) for c in range(n)]
+    u = [rho, *top[:3], en, *top[3:]]
+    for c in (1, 2, 3, 5, 6, 7, 8)[:n]:
+        small = 2.0 ** rng.uniform(tiny + 0.01, np.maximum(np.log2(u[c]), tiny + 0.02))
+        kind = rng.random(shape)
+        u[c] = np.where(kind < 0.25, 0.0, np.where(kind < 0.5, 2.0 ** (tiny + 0.01), np.where(kind < 0.75, small, u[c])))
+        u[c] *= rng.choice([-1.0, 1.0], shape)
+    return np.ascontiguousarray(np.stack(u))
+
+
+@pytest.mark.parametrize("faces", ["default", "rusanov"])
+@pytest.mark.parametrize("mhd", [False, True])
+@pytest.mark.parametrize("name", ["13x13x11", "open", "forest"])
+def test_states_inside_the_domain(name, mhd, faces):
+    m = MESHES[name]()
+    kw = dict(positivity=0, indicator=abi.IND_MODAL)
+    if mhd:
+        kw.update(eqn=abi.EQN_MHD, n_vars=9, kappa=5.0 / 3.0, volume_flux=abi.VOLFLUX_EC_MHD, surface_flux=abi.SURFFLUX_HLLD,
+                  glm_ch=0.7, glm_alpha=0.3)
+    if faces == "rusanov":
+        kw.update(surface_flux=abi.SURFFLUX_RUSANOV, volume_flux=abi.VOLFLUX_CENTRAL)
+    c = abi.default_cfg(**kw)
+    s = Solver(c, m)
+    o = orc.Oracle.for_mesh(c, m)
+    for seed in range(3):
+        u = corners(np.random.default_rng(seed), (m.E, 64), mhd)
+        assert np.isfinite(u).all()
+        s.upload(u)
+        assert np.array_equal(s.rhs(), o.rhs(u, alpha=o.alpha(u)), equal_nan=True), seed
