@@ -34,8 +34,8 @@ namespace {
 // (96 registers and 1 KB of spills, 18 warps per SM, instruction fetch the second largest stall).  As
 // tasks the kernel holds one copy of each flux, and no element waits for another of its CTA.  With the
 // quotients of ieee64.cuh, B200, us per stage, line form -> this: Sedov 32^3 664 -> 381 (0.16 of the FP64
-// FMA peak by algorithmic flops), Kelvin-Helmholtz forest of 24k elements 619 -> 340, 4^3 elements
-// 38 -> 19 (with the compiler's quotients and 16 warps per SM the task form alone was 727 at 32^3).
+// FMA peak by algorithmic flops; 392 with the check of their domain), Kelvin-Helmholtz forest of 24k elements
+// 619 -> 340, 4^3 elements 38 -> 19 (with the compiler's quotients and 16 warps per SM the task form alone was 727 at 32^3).
 // What bounds it now (ncu, Sedov 32^3): 242 M warp instructions at 56 % issue, of which 103 M FP64 (the
 // FP64 pipe 49 % busy); stalls per issue: dependent latency 2.3, CTA barriers 1.5, instruction fetch 1.2.
 // Resident elements per SM at 14 / 12 / 10 / 8 (72, 80, 96, 128 registers): 424 / 397 / 403 / 420 us
@@ -738,7 +738,8 @@ static int smem64(int nd, bool blend) {
 // Up to so many elements, what the SMs hold at once with ND = 1, three directions at a time (set by the setup).
 // B200, us per stage, blended: 64 elements 14.3 -> 9.2, 216 15.0 -> 10.6, 512 17 -> 14, 910 22.6 -> 21.6, 1584
 // 31.0 -> 30.5; beyond, the wider CTAs' idle warps cost more than they save: 2197 39.1 -> 39.2, 4096 59.6 -> 65.8,
-// 32768 380 -> 491.
+// 32768 380 -> 491.  With the check of the quotients' domain, smooth flow (few blended elements): 64 14.9 -> 9.6, 216
+// 15.9 -> 11.7, 512 18.9 -> 15.5, 910 25.3 -> 24.2, 1584 26.4 -> 27.8, 4096 52.2 -> 63.1.
 static int64_t wide_elems64 = 0;
 
 template <int ND>
